@@ -98,9 +98,9 @@ def build_reference(verbose=False, force=False, ref_root=None):
     """Compiles the reference's CUDA sources (never copied) with oracle/build_ref.py,
     and the reference's driver against the drop-in headers (oracle/_ref/slak_main_dropin).
     The reference tree is `ref_root`, else $SLAK_REFERENCE_ROOT; with neither
-    (or no such directory) nothing is built and None is returned."""
+    (or no sources in that directory) nothing is built and None is returned."""
     ref_root = ref_root or os.environ.get("SLAK_REFERENCE_ROOT")
-    if not ref_root or not os.path.isdir(ref_root):
+    if not ref_root or not os.path.isdir(os.path.join(ref_root, "LibSource", "device")):
         return None
     sys.path.insert(0, _paths.REPO_DIR)
     try:
