@@ -419,7 +419,7 @@ __device__ __forceinline__ void gq_columns(const FastDims& d, QState& c, const f
 }
 
 // ---------------------------------------------------------------------------------------------
-// SG: the last level with P = refine(PP), PP a closed quad mesh; `pp` is PP's
+// SG: the last GQ level (P = refine(PP), PP a closed quad mesh); `pp` is PP's
 // state, and the level before writes none.  P's twin, slot and (SLAK) t of
 // corner x = 4y + k are what write_state would have stored, from PP's twin of
 // y (of prev(y) for k = 3), PP's slot and t of y (k = 0) and, for k = 1, 3,
@@ -580,6 +580,8 @@ __device__ __forceinline__ void k_g1_body(const unsigned bx_, FastDims d, Faces<
             st8_cs(dst, make_int4(Q.x, VFc + e0, fpid, VFc + e3), make_int4(Q.y, VFc + e1, fpid, VFc + e0));
             st8_cs(dst + 2, make_int4(Q.z, VFc + e2, fpid, VFc + e1), make_int4(Q.w, VFc + e3, fpid, VFc + e2));
         }
+    } else if (out_ids == nullptr) {
+        // the next level takes its quads from this level's input
     } else if constexpr (kTmaQuadStore && BS <= 256) {
         // the block's refined quads (row t = thread t's 64 bytes) staged in
         // shared memory in the tensor map's 64-byte swizzle (16-byte chunk k
@@ -1114,10 +1116,26 @@ __device__ __forceinline__ void g3_small(const FastDims& d, const float* __restr
     if (STATE) c.sptr[v] = b;
 }
 
+// The record of slot s: the face point, and the neighbour position.  PP levels
+// (grand.cuh) store SLAK records as the face point alone: the neighbour, on
+// the P edge whose id is the slot, is C's vertex V1 + F1 + s.
+template <bool LAK, bool PP>
+__device__ __forceinline__ float4 rec_f(const float4* __restrict__ Z, int64_t s)
+{
+    return __ldg(Z + (PP && !LAK ? s : 2 * s));
+}
+template <bool LAK, bool PP>
+__device__ __forceinline__ float4 rec_n(const FastDims& d, const float* __restrict__ P, const float4* __restrict__ Z,
+                                        int64_t s)
+{
+    if constexpr (PP && !LAK) return ldg4(P, d.V1 + d.F1 + s);
+    else return __ldg(Z + 2 * s + 1);
+}
+
 // ---------------------------------------------------------------------------------------------
 // One vertex of P on its own thread (columns of up to kBigCol slots, and
 // columns too long for the warp path).
-template <bool LAK, bool STATE, bool BND>
+template <bool LAK, bool STATE, bool BND, bool PP = false>
 __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ P, QState c, SlotScratch z,
                                           float* __restrict__ R, int compensated, int v, int b, int n)
 {
@@ -1135,7 +1153,8 @@ __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ 
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (k < n) {
-                ld8_nc(Z + 2 * (int64_t)(b + k), zf[k], zn[k]);
+                if constexpr (PP && !LAK) { zf[k] = rec_f<LAK, PP>(Z, b + k); zn[k] = rec_n<LAK, PP>(d, P, Z, b + k); }
+                else ld8_nc(Z + 2 * (int64_t)(b + k), zf[k], zn[k]);
                 tt[k] = LAK ? __ldg(z.T + b + k) : __ldg(z.rot + b + k) - b;
                 if (BND) fl[k] = __ldg(z.bflag + b + k);
             }
@@ -1144,8 +1163,8 @@ __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ 
         return;
     }
     const bool comp = compensated && n > 4;
-    const auto zf = [&](int k) { return __ldg(Z + 2 * (int64_t)(b + k)); };        // FP(x) of slot b+k
-    const auto zn = [&](int k) { return __ldg(Z + 2 * (int64_t)(b + k) + 1); };    // its neighbour
+    const auto zf = [&](int k) { return rec_f<LAK, PP>(Z, b + k); };          // FP(x) of slot b+k
+    const auto zn = [&](int k) { return rec_n<LAK, PP>(d, P, Z, b + k); };    // its neighbour
     if (!LAK) {
         if (!comp) {
             float4 acc = f4_zero();
@@ -1161,7 +1180,7 @@ __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ 
         // edge points of C's edges {v, e_out(x)}, ids b..e-1:
         // 0 + (p_v + FP(x))/4 + (Z[2s+1] + Z[2 rot[s]])/4
         const int64_t EPb = (int64_t)d.V + d.N1;
-        for_each_loaded(n, [&](int k) { return f4_add(zn(k), __ldg(Z + 2 * (int64_t)__ldg(z.rot + b + k))); },
+        for_each_loaded(n, [&](int k) { return f4_add(zn(k), rec_f<LAK, PP>(Z, __ldg(z.rot + b + k))); },
                         [&](int k, float4 t) {
                             if (BND && (__ldg(z.bflag + b + k) & 1)) {
                                 st4_cs(R, EPb + b + k, f4_mul(f4_add(Pv, zn(k)), 0.5f));
@@ -1188,7 +1207,7 @@ __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ 
                     if (ti > last && ti < xm) { xm = ti; sm = s; }
                 }
                 if (sm < 0) break;
-                const float4 pt = __ldg(Z + 2 * (int64_t)sm + 1);
+                const float4 pt = rec_n<LAK, PP>(d, P, Z, sm);
                 if (comp) dd_acc(sh, sl, pt); else acc = f4_add(acc, pt);
                 last = xm;
             }
@@ -1207,7 +1226,7 @@ __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ 
 // slot; the sums run in the order the single-thread path uses, every lane
 // fetching slot k (or the tail of rank r) by shuffle, so the result is the
 // same bit for bit.  No shared memory: the common path keeps its L1.
-template <bool LAK, bool STATE, bool BND>
+template <bool LAK, bool STATE, bool BND, bool PP = false>
 __device__ __noinline__ void g3_warp_column(FastDims d, const float* __restrict__ P, QState c, SlotScratch z,
                                             float* __restrict__ R, int compensated, int v, int b, int n)
 {
@@ -1218,8 +1237,8 @@ __device__ __noinline__ void g3_warp_column(FastDims d, const float* __restrict_
     float4 f0 = f4_zero(), f1 = f4_zero(), n0 = f4_zero(), n1 = f4_zero();   // FP(x) and the neighbour
     int t0 = INT32_MAX, t1 = INT32_MAX;
     // two 16-byte loads per record here: ptxas 12.9 fails on the 256-bit load in this function
-    if (h0) { f0 = __ldg(Z + 2 * (int64_t)k0); n0 = __ldg(Z + 2 * (int64_t)k0 + 1); if (LAK) t0 = __ldg(z.T + k0); }
-    if (h1) { f1 = __ldg(Z + 2 * (int64_t)k1); n1 = __ldg(Z + 2 * (int64_t)k1 + 1); if (LAK) t1 = __ldg(z.T + k1); }
+    if (h0) { f0 = rec_f<LAK, PP>(Z, k0); n0 = rec_n<LAK, PP>(d, P, Z, k0); if (LAK) t0 = __ldg(z.T + k0); }
+    if (h1) { f1 = rec_f<LAK, PP>(Z, k1); n1 = rec_n<LAK, PP>(d, P, Z, k1); if (LAK) t1 = __ldg(z.T + k1); }
     const float4 Pv = ldg4(P, v);
     if (!LAK) {
         // edge points of C's edges {v, e_out(x)}, ids b..e-1: 0 + (p_v + FP(x))/4 + (Z[2s+1] + Z[2 rot[s]])/4,
@@ -1287,44 +1306,55 @@ __device__ __noinline__ void g3_warp_column(FastDims d, const float* __restrict_
 // boundary (BND), an edge {v, e_out(x)} without a twin gets the midpoint.
 // Columns longer than kBigCol go to their warp (g3_warp_column).
 // `nv`: the vertices of P it covers, V1 (or V2 on a GQ level, whose other
-// columns k_g1 sums).
-template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false>
+// columns k_g1 sums).  PP (grand.cuh): `p` is PP's state and the vertices are
+// PP's V2 old ones, which keep their columns, then, for a polygon PP (`pptr`
+// its face offsets), the F2 face points, of which the long faces' are summed
+// here.
+template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false, bool PP = false>
 __device__ __forceinline__ void k_g3_body(const unsigned bx_, FastDims d, const float* __restrict__ P, QState p, QState c,
-                                          SlotScratch z, float* __restrict__ R, int compensated, int nv)
+                                          SlotScratch z, float* __restrict__ R, int compensated, int nv,
+                                          const int* __restrict__ pptr, int ppface)
 {
     const int v = bx_ * blockDim.x + threadIdx.x;
     if (STATE && v == nv) c.sptr[d.V] = d.N;
-    const bool valid = v < nv;
+    bool valid = v < nv;
     int b = 0, n = 0;
     if (valid) {
         if constexpr (SG) { b = sg_sptr(d, p.sptr, v); n = sg_sptr(d, p.sptr, v + 1) - b; }
+        else if (PP && v >= d.V2) {
+            b = __ldg(pptr + v - d.V2);
+            n = __ldg(pptr + v - d.V2 + 1) - b;
+            b += d.N2;
+            valid = n > ppface;
+        }
         else { b = __ldg(p.sptr + v); n = __ldg(p.sptr + v + 1) - b; }
     }
     const bool big = valid && n > kBigCol && n <= kWarpCol;
-    if (valid && !big) g3_vertex<LAK, STATE, BND>(d, P, c, z, R, compensated, v, b, n);
+    if (valid && !big) g3_vertex<LAK, STATE, BND, PP>(d, P, c, z, R, compensated, v, b, n);
     unsigned m = __ballot_sync(0xffffffffu, big);
     while (m) {
         const int src = __ffs(m) - 1;
         m &= m - 1;
-        g3_warp_column<LAK, STATE, BND>(d, P, c, z, R, compensated, __shfl_sync(0xffffffffu, v, src),
-                                        __shfl_sync(0xffffffffu, b, src), __shfl_sync(0xffffffffu, n, src));
+        g3_warp_column<LAK, STATE, BND, PP>(d, P, c, z, R, compensated, __shfl_sync(0xffffffffu, v, src),
+                                            __shfl_sync(0xffffffffu, b, src), __shfl_sync(0xffffffffu, n, src));
     }
 }
-template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false>
+template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false, bool PP = false>
 __global__ void __launch_bounds__(BS) k_g3(FastDims d, const float* __restrict__ P, QState p, QState c,
-                                           SlotScratch z, float* __restrict__ R, int compensated, int nv)
+                                           SlotScratch z, float* __restrict__ R, int compensated, int nv,
+                                           const int* __restrict__ pptr, int ppface)
 {
     griddep_enter();
-    k_g3_body<LAK, STATE, BS, BND, SG>(blockIdx.x, d, P, p, c, z, R, compensated, nv);
+    k_g3_body<LAK, STATE, BS, BND, SG, PP>(blockIdx.x, d, P, p, c, z, R, compensated, nv, pptr, ppface);
 }
-template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false>
+template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false, bool PP = false>
 struct k_g3_g {
     static constexpr int kBounds = 1, kMaxT = BS, kMinB = 0;
     template <class... A> __device__ __forceinline__ void operator()(unsigned bx, const A&... a) const
     {
-        k_g3_body<LAK, STATE, BS, BND, SG>(bx, a...);
+        k_g3_body<LAK, STATE, BS, BND, SG, PP>(bx, a...);
     }
-    static constexpr auto kernel() { return &k_g3<LAK, STATE, BS, BND, SG>; }
+    static constexpr auto kernel() { return &k_g3<LAK, STATE, BS, BND, SG, PP>; }
 };
 
 // ---------------------------------------------------------------------------------------------

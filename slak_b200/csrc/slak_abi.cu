@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "general.cuh"
 #include "fast.cuh"
+#include "grand.cuh"
 #include "scan.cuh"
 #include "crease.cuh"
 
@@ -45,10 +46,13 @@ struct Level {
     // k_g1 sums most of the parent's vertex columns; that mesh's sizes
     bool gq = false;
     int64_t gN = 0, gV = 0, gF = 0;
-    // the last level, when its parent's parent is a closed quad mesh (SG,
-    // fast.cuh): it takes its parent's state in closed form from the
-    // grandparent's, so the level before writes none
+    // the last GQ level: it takes its parent's state in closed form from the
+    // grandparent's (SG, fast.cuh), so the level before writes none
     bool sg = false;
+    // closed level with a grandparent (grand.cuh): refined from the
+    // grandparent's state and the parent's quads
+    bool pp = false;
+    bool skip_ids = false;       // its refined quads are read by no later level
     // k_g3 with bulk-copied slot records (SLAK_PLAN_BULK_RECORDS, closed parents)
     bool bulk3 = false;
     int bulk_polls = 0;
@@ -179,19 +183,19 @@ struct slak_plan {
     // device memory
     void* arena = nullptr;
     Scratch s;
-    int* ping_ids[2] = {nullptr, nullptr};
-    float* ping_verts[2] = {nullptr, nullptr};
+    std::vector<int*> mid_ids;       // intermediate meshes, per level (null: not written)
+    std::vector<float*> mid_verts;
     DevStatus* st = nullptr;
     DevStatus* h_st = nullptr;       // pinned
     bool h_st_owned = true;
     int64_t maxN = 0, maxV = 0, maxE = 0;
     bool any_poly = false;
-    int64_t exN = 0, stN = 0, stV = 0, slN = 0, mid_ids = 0, mid_verts = 0;
-    int64_t exE = 0, stE = 0;        // edges of the exported / state levels (boundary ranks)
+    int64_t exN = 0, slN = 0;
+    int64_t exE = 0;                 // edges of the exported level (boundary ranks)
     bool bnd_fast = false;           // some fast level has a parent with a boundary
     int* bnd_tmp = nullptr;          // scan tiles for C's boundary ranks
     bool arena_owned = true;
-    QState qs[2]{};
+    std::vector<QState> qs;          // adjacency state a fast level writes, per level
     SlotScratch slots{};
     // graph
     cudaGraphExec_t gexec = nullptr;
@@ -372,11 +376,7 @@ void launch_rest(const Level& L, int li, int scheme, bool compensated, Scratch& 
     if (lc.conc) { lc.join(0); lc.join(1); }
 }
 
-// The tensor map of a level's refined quads for k_g1's tensor store: `rows`
-// rows of 16 int32 (thread x's four quads at out + 16 x), boxes of `bs` rows,
-// 64-byte swizzle (the layout k_g1 stages them in).  A null `out` (a launch
-// sequence recorded before any memory exists) leaves the map zeroed.
-bool quad_store_map(CUtensorMap& m, int* out, int64_t rows, int bs)
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 {
     static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
     static std::once_flag once;
@@ -387,6 +387,16 @@ bool quad_store_map(CUtensorMap& m, int* out, int64_t rows, int bs)
             q == cudaDriverEntryPointSuccess)
             enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
     });
+    return enc;
+}
+
+// The tensor map of a level's refined quads for k_g1's tensor store: `rows`
+// rows of 16 int32 (thread x's four quads at out + 16 x), boxes of `bs` rows,
+// 64-byte swizzle (the layout k_g1 stages them in).  A null `out` (a launch
+// sequence recorded before any memory exists) leaves the map zeroed.
+bool quad_store_map(CUtensorMap& m, int* out, int64_t rows, int bs)
+{
+    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (out == nullptr) return true;
     if (enc == nullptr || rows < 1) {
         g_detail = "cuTensorMapEncodeTiled unavailable";
@@ -403,6 +413,28 @@ bool quad_store_map(CUtensorMap& m, int* out, int64_t rows, int bs)
     return r == CUDA_SUCCESS;
 }
 
+// The same of a PP level (grand.cuh): thread y's 256 bytes as two rows of 128
+// (halves of one row of 64 int32), boxes of one half of `bs` threads, 128-byte
+// swizzle.
+bool quad_store_map2(CUtensorMap& m, int* out, int64_t rows, int bs)
+{
+    if (out == nullptr) return true;
+    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    if (enc == nullptr || rows < 1) {
+        g_detail = "cuTensorMapEncodeTiled unavailable";
+        return false;
+    }
+    const cuuint64_t dims[3] = {32, 2, (cuuint64_t)rows};
+    const cuuint64_t strides[2] = {128, 256};
+    const cuuint32_t box[3] = {32, 1, (cuuint32_t)bs};
+    const cuuint32_t es[3] = {1, 1, 1};
+    const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, out, dims, strides, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) g_detail = "cuTensorMapEncodeTiled: error " + std::to_string((int)r);
+    return r == CUDA_SUCCESS;
+}
+
 // One fast level: C = L (refined from its parent level Pl, whose state is
 // L.in_state).  BND: Pl has a boundary (quad faces only).
 template <bool LAK, bool STATE, bool PQ, bool BND, bool GQ = false, bool SG = false>
@@ -414,7 +446,7 @@ void launch_fast_t(const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc&
     cudaStream_t str = lc.s;
     // compulsory bytes of each kernel: the level's corner ids and positions it
     // must read once, and the refined ids / positions it alone writes
-    const int64_t g1b = 4 * L.N + 16 * L.V + 16 * L.N + 16 * L.F + 16 * Pl.F + (LAK ? 0 : 16 * L.F);
+    const int64_t g1b = 4 * L.N + 16 * L.V + (L.skip_ids ? 0 : 16 * L.N) + 16 * L.F + 16 * Pl.F + (LAK ? 0 : 16 * L.F);
     const int64_t g2b = 16 * Pl.E + (LAK ? 16 * 2 * L.F : 0);
     // LAK's last level: the refined ptr / vals come from k_g1 too
     int* optr = LAK && !STATE ? L.o_ptr : nullptr;
@@ -454,7 +486,7 @@ void launch_fast_t(const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc&
     } else {
         with_block(L.bs[2], [&](auto b) {
             constexpr int BS = decltype(b)::value;
-            launch_g<k_g3_g<LAK, STATE, BS, BND, SG>>(grid_for(nv3 + 1, BS), BS, str, d, L.verts, L.in_state, L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv3);
+            launch_g<k_g3_g<LAK, STATE, BS, BND, SG>>(grid_for(nv3 + 1, BS), BS, str, d, L.verts, L.in_state, L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv3, nullptr, 0);
         });
     }
     // compulsory bytes: the vertex points of its vertices, SLAK the edge points of their slots
@@ -471,7 +503,7 @@ void launch_fast_t(const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc&
 template <bool PQ, bool BND, bool GQ = false>
 void launch_fast_p(const Level& Pl, const Level& L, Faces<PQ> pf, bool lak, bool comp, Lc& lc)
 {
-    if constexpr (PQ && !BND) {
+    if constexpr (GQ) {
         if (L.sg) {             // the last level: no state to write
             if (lak) launch_fast_t<true, false, PQ, BND, GQ, true>(Pl, L, pf, comp, lc);
             else launch_fast_t<false, false, PQ, BND, GQ, true>(Pl, L, pf, comp, lc);
@@ -487,12 +519,72 @@ void launch_fast_p(const Level& Pl, const Level& L, Faces<PQ> pf, bool lak, bool
     }
 }
 
-// `cface` is the parent's corner -> face map when the parent is a polygon level
-void launch_fast(const Level& Pl, const Level& L, const int* cface, int scheme, bool comp, Lc& lc)
+// One PP level (grand.cuh): C = L, its parent Pl and its parent's parent PPl,
+// whose state is L.in_state.  The block size bs[0] counts C's quads: four per
+// thread of k_pp.
+template <bool LAK, bool STATE, bool PQ>
+void launch_pp_t(const Level& PPl, const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc& lc)
 {
+    FastDims d{(int)Pl.N, (int)Pl.V, (int)Pl.F, (int)Pl.E, (int)L.V, (int)L.N, 0};
+    d.N2 = (int)PPl.N; d.V2 = (int)PPl.V; d.F2 = (int)PPl.F;
+    int* optr = LAK && !STATE ? L.o_ptr : nullptr;
+    int4* ovals = LAK && !STATE ? reinterpret_cast<int4*>(L.o_vals) : nullptr;
+    const int wids = L.skip_ids ? 0 : 1;
+    bool mapped = true;
+    with_block(L.bs[0], [&](auto b) {
+        constexpr int BS = decltype(b)::value / 4;
+        CUtensorMap otm;
+        std::memset(&otm, 0, sizeof otm);
+        if (wids) mapped = quad_store_map2(otm, L.o_ids, PPl.N, BS);
+        if (!mapped) return;            // nothing of the level is launched
+        launch_g<k_pp_g<LAK, STATE, PQ, BS>>(grid_for(PPl.N, BS), BS, lc.s, d, pf, reinterpret_cast<const int4*>(Pl.ids),
+                                             L.verts, L.in_state, L.out_state, wids, otm, L.o_verts, L.slots, optr,
+                                             ovals, comp ? 1 : 0);
+    });
+    if (!mapped) {
+        if (!lc.err) lc.err = SLAK_ERR_CUDA;
+        return;
+    }
+    // compulsory bytes: the parent's quads and C's positions in; the refined
+    // quads, all refined positions but k_g3's out
+    const int64_t g3 = 16 * PPl.V + (LAK ? 0 : 16 * PPl.N);
+    lc.after("k_pp", 1, 16 * PPl.N + 16 * L.V + (wids ? 16 * L.N : 0) + 16 * L.Vo - g3 +
+                            (optr ? 4 * (L.N + 1) + 16 * L.N : 0));
+    const int nv = (int)(PQ ? PPl.V : PPl.V + PPl.F);
+    with_block(L.bs[2], [&](auto b) {
+        constexpr int BS = decltype(b)::value;
+        launch_g<k_g3_g<LAK, STATE, BS, false, false, true>>(grid_for(nv + 1, BS), BS, lc.s, d, L.verts, L.in_state,
+                                                             L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv,
+                                                             PQ ? nullptr : PPl.ptr, kPpFace);
+    });
+    lc.after("k_g3", 1, g3);
+}
+
+template <bool PQ>
+void launch_pp(const Level& PPl, const Level& Pl, const Level& L, Faces<PQ> pf, bool lak, bool comp, Lc& lc)
+{
+    if (lak) {
+        if (L.make_state) launch_pp_t<true, true, PQ>(PPl, Pl, L, pf, comp, lc);
+        else launch_pp_t<true, false, PQ>(PPl, Pl, L, pf, comp, lc);
+    } else {
+        if (L.make_state) launch_pp_t<false, true, PQ>(PPl, Pl, L, pf, comp, lc);
+        else launch_pp_t<false, false, PQ>(PPl, Pl, L, pf, comp, lc);
+    }
+}
+
+// `L` is the level, L[-1] its parent; `cface` is level 0's corner -> face map
+// when it has polygon faces
+void launch_fast(const Level* Lp, const int* cface, int scheme, bool comp, Lc& lc)
+{
+    const Level &L = *Lp, &Pl = Lp[-1];
     const bool lak = scheme == SLAK_SCHEME_LAK;
+    if (L.pp) {
+        const Level& PPl = Lp[-2];
+        if (PPl.quad) launch_pp<true>(PPl, Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
+        else launch_pp<false>(PPl, Pl, L, Faces<false>{PPl.ptr, cface}, lak, comp, lc);
+        return;
+    }
     if (L.gq) launch_fast_p<true, false, true>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
-    else if (L.sg) launch_fast_p<true, false>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
     else if (Pl.quad && Pl.B > 0) launch_fast_p<true, true>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
     else if (Pl.quad) launch_fast_p<true, false>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
     else if (Pl.B > 0) launch_fast_p<false, true>(Pl, L, Faces<false>{Pl.ptr, cface}, lak, comp, lc);
@@ -574,7 +666,7 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
         const Level& L = p->lv[li];
         lc.level = (int)li;
         if (L.fast) {
-            launch_fast(p->lv[li - 1], L, p->s.cface, p->scheme, comp, lc);
+            launch_fast(&L, p->s.cface, p->scheme, comp, lc);
             if (lc.err) break;          // a level that could not be launched stops the plan
             if ((int)li < p->crease_levels) launch_creases(p, (int)li, lc);
             continue;
@@ -723,14 +815,17 @@ int plan_levels(slak_plan* p)
         }
         L.Fo = L.N; L.No = 4 * L.N; L.Vo = L.V + L.F + L.E;
         if (L.No >= (1ll << 31) || L.Vo >= (1ll << 31)) return SLAK_ERR_UNSUPPORTED;
-        // the parent is refine(PP) with PP a closed quad mesh: GQ on request; SG
-        // on the last level (SLAK_NO_SG builds: off, for comparisons)
-        const bool gq_parent = L.fast && i >= 2 && p->lv[i - 2].quad && p->lv[i - 2].B == 0;
-        if (gq_parent && (p->flags & SLAK_PLAN_GQ)) L.gq = true;
-#ifndef SLAK_NO_SG
-        if (gq_parent && i == nlev - 1 && p->lv[i - 1].fast) L.sg = true;
-#endif
-        if (L.gq || L.sg) { L.gN = p->lv[i - 2].N; L.gV = p->lv[i - 2].V; L.gF = p->lv[i - 2].F; }
+        // the parent is refine(PP) with PP closed: refined from PP's state
+        // (grand.cuh), unless a layout kept for comparison is asked for: GQ (PP
+        // with quad faces; SG on the last level) or bulk-copied records
+        if (L.fast && i >= 2 && p->lv[i - 2].B == 0) {
+            if (!(p->flags & (SLAK_PLAN_GQ | SLAK_PLAN_BULK_RECORDS))) L.pp = true;
+            else if ((p->flags & SLAK_PLAN_GQ) && p->lv[i - 2].quad) {
+                L.gq = true;
+                L.sg = i == nlev - 1;
+                L.gN = p->lv[i - 2].N; L.gV = p->lv[i - 2].V; L.gF = p->lv[i - 2].F;
+            }
+        }
         if (!L.fast) {
             if (L.N > p->maxN) p->maxN = L.N;
             if (L.V > p->maxV) p->maxV = L.V;
@@ -752,16 +847,16 @@ int plan_levels(slak_plan* p)
             if (L.N > p->exN) p->exN = L.N;
             if (L.B > 0 && L.E > p->exE) p->exE = L.E;
         }
-        if (L.fast && i + 1 < nlev && p->lv[i + 1].fast && !p->lv[i + 1].sg) {
-            L.make_state = true;
-            if (L.N > p->stN) p->stN = L.N;
-            if (L.V > p->stV) p->stV = L.V;
-            if (L.B > 0 && L.E > p->stE) p->stE = L.E;
+        // the state of the level's input is read by the next level, or by the
+        // one after it when that is a PP level
+        if (L.fast && i + 1 < nlev) {
+            const Level& n1 = p->lv[i + 1];
+            if (!n1.sg && !n1.pp) L.make_state = true;
+            if (i + 2 < nlev && p->lv[i + 2].pp) L.make_state = true;
         }
-    }
-    for (int i = 0; i + 1 < nlev; ++i) {
-        if (p->lv[i].No > p->mid_ids) p->mid_ids = p->lv[i].No;
-        if (p->lv[i].Vo > p->mid_verts) p->mid_verts = p->lv[i].Vo;
+        // the last level's own quads are read by no one when it is a PP level
+        // (the crease passes read every mesh's)
+        L.skip_ids = i == nlev - 2 && p->lv[i + 1].pp;
     }
     return SLAK_OK;
 }
@@ -773,9 +868,10 @@ void plan_carve(slak_plan* p, Carver& cv)
     const int nlev = (int)p->lv.size();
     carve_scratch(cv, p->s, p->maxN, p->maxV, p->maxE, p->any_poly);
     if (p->exN) carve_export(cv, p->s, p->exN, p->exE);
-    if (p->stN) {
-        carve_state(cv, p->qs[0], p->stN, p->stV, p->stE);
-        carve_state(cv, p->qs[1], p->stN, p->stV, p->stE);
+    p->qs.assign(nlev, QState{});
+    for (int i = 0; i < nlev; ++i) {
+        const Level& L = p->lv[i];
+        if (L.make_state) carve_state(cv, p->qs[i], L.N, L.V, L.B > 0 ? L.E : 0);
     }
     if (p->slN) {
         p->slots.Z = cv.take<float4>(2 * p->slN);
@@ -787,9 +883,11 @@ void plan_carve(slak_plan* p, Carver& cv)
             p->bnd_tmp = cv.take<int>(scan_tiles(p->slN) + 2);
         }
     }
-    for (int k = 0; k < 2; ++k) {
-        p->ping_ids[k] = nlev > 1 ? cv.take<int>(p->mid_ids) : nullptr;
-        p->ping_verts[k] = nlev > 1 ? cv.take<float>(4 * p->mid_verts) : nullptr;
+    p->mid_ids.assign(nlev, nullptr);
+    p->mid_verts.assign(nlev, nullptr);
+    for (int i = 0; i + 1 < nlev; ++i) {
+        if (!p->lv[i].skip_ids) p->mid_ids[i] = cv.take<int>(p->lv[i].No);
+        p->mid_verts[i] = cv.take<float>(4 * p->lv[i].Vo);
     }
     p->st = cv.take<DevStatus>(1);
     if (p->crease_levels > 0) {
@@ -840,18 +938,18 @@ void plan_wire(slak_plan* p)
             L.o_ids = p->out.ids; L.o_verts = p->out.verts;
             L.o_ptr = p->out.ptr; L.o_vals = p->out.vals;
         } else {
-            L.o_ids = p->ping_ids[i & 1]; L.o_verts = p->ping_verts[i & 1];
+            L.o_ids = p->mid_ids[i]; L.o_verts = p->mid_verts[i];
         }
     }
-    int qi = 0;
     for (int i = 1; i < nlev; ++i) {
         Level& L = p->lv[i];
         if (!L.fast) continue;
         const Level& P = p->lv[i - 1];
-        if (L.sg) L.in_state = P.in_state;      // the grandparent's state: the parent's own input
-        else if (P.export_state) L.in_state = QState{p->s.sptr, p->s.xslot, p->s.xtw, p->s.xt, p->s.xbrank};
-        else L.in_state = P.out_state;
-        if (L.make_state) { L.out_state = p->qs[qi]; qi ^= 1; }
+        // the parent's state, or (SG, PP) the grandparent's
+        const Level& S = p->lv[L.sg || L.pp ? i - 2 : i - 1];
+        if (S.export_state) L.in_state = QState{p->s.sptr, p->s.xslot, p->s.xtw, p->s.xt, p->s.xbrank};
+        else L.in_state = S.out_state;
+        if (L.make_state) L.out_state = p->qs[i];
         L.slots = p->slots;
         L.scan_tmp = p->bnd_tmp;
         L.st = p->st;
@@ -940,7 +1038,7 @@ std::string tune_key(const slak_plan* p, int li)
     char buf[96];
     std::snprintf(buf, sizeof buf, "%s/%s%s/%s/q2^%d/vmax%d/v4_%d", p->scheme == SLAK_SCHEME_LAK ? "lak" : "slak",
                   L.gq ? "gquad" : P.quad ? "quad" : "poly", P.B > 0 ? "-open" : "",
-                  L.make_state ? "state" : L.sg ? "last-sg" : "last",
+                  L.pp ? (L.make_state ? "pp-state" : "pp-last") : L.make_state ? "state" : L.sg ? "last-sg" : "last",
                   fb, vclass, sclass);
     return buf;
 }
@@ -1027,7 +1125,7 @@ int plan_autotune(slak_plan* p, cudaStream_t str)
                 for (int r = 0; r < 3 && rc == SLAK_OK; ++r) {
                     rc = enqueue_all(p, str);
                     if (rc == SLAK_OK) rc = cuda_status(cudaStreamSynchronize(str));
-                    t[r] = kernel_ms(p, li, kTuneKernels[k]);
+                    t[r] = kernel_ms(p, li, k == 0 && L.pp ? "k_pp" : kTuneKernels[k]);
                 }
                 std::sort(t, t + 3);
                 L.tune_ms[k][ci] = t[1];
@@ -1124,6 +1222,7 @@ static int plan_create_impl(const slak_mesh* cm, int target_level, int scheme, i
     }
     if (rc == SLAK_OK && (ncrease > 0 || ncorner > 0))
         rc = plan_crease_setup(p, csharp, ncrease, kverts, ksharp, ncorner, str);
+    for (int i = 0; i < p->crease_levels; ++i) p->lv[i].skip_ids = false;
     if (rc != SLAK_OK) { free_plan_memory(p); delete p; return rc; }
     Carver dry(nullptr);
     plan_carve(p, dry);
