@@ -12,17 +12,22 @@ Run ``python -m slak_b200.build`` or ``__graft_entry__.build()``.
 """
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import shutil
 import subprocess
 import sys
+import tempfile
 
 from . import _paths
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc" if os.path.exists("/usr/local/cuda/bin/nvcc") else "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUDA_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC",
-                     "-Xcompiler", "-O3", "--expt-relaxed-constexpr"]
+                     "-Xcompiler", "-O3", "--expt-relaxed-constexpr", "--compress-mode=size"]
+
+
+LEVEL_UNITS = range(1, 8)
 
 
 def _run(cmd, verbose):
@@ -50,14 +55,21 @@ def _csrc(*names):
 
 def build_cuda(verbose=False, force=False, extra=None):
     os.makedirs(_paths.LIB_DIR, exist_ok=True)
-    srcs = _csrc("slak_abi.cu") + _csrc("objio.cpp")
+    srcs = _csrc("slak_abi.cu", "levels.cu", "objio.cpp")
     deps = srcs + [os.path.join(_paths.CSRC_DIR, f) for f in os.listdir(_paths.CSRC_DIR)
                    if f.endswith((".cuh", ".h"))] + [os.path.join(_paths.INCLUDE_DIR, "slak_b200.h")]
     if not force and not _stale(_paths.LIB_SLAK, deps):
         return _paths.LIB_SLAK
-    cmd = [NVCC] + CUDA_FLAGS + (extra or []) + ["-shared", "-I", _paths.INCLUDE_DIR, "-I", _paths.CSRC_DIR,
-                                                 "-o", _paths.LIB_SLAK] + srcs
-    _run(cmd, verbose)
+    # the units of levels.cu (one kind of level each) beside the rest, then one link
+    flags = CUDA_FLAGS + (extra or []) + ["-I", _paths.INCLUDE_DIR, "-I", _paths.CSRC_DIR]
+    units = [("levels.cu", [f"-DSLAK_UNIT={k}"], f"levels{k}.o") for k in LEVEL_UNITS]
+    units += [("slak_abi.cu", [], "slak_abi.o"), ("objio.cpp", [], "objio.o")]
+    with tempfile.TemporaryDirectory() as odir:
+        objs = [os.path.join(odir, o) for _, _, o in units]
+        with concurrent.futures.ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+            list(pool.map(lambda u: _run([NVCC] + flags + u[0][1] + ["-c", "-o", u[1]] + _csrc(u[0][0]), verbose),
+                          zip(units, objs)))
+        _run([NVCC] + ARCH + ["-shared", "-o", _paths.LIB_SLAK] + objs, verbose)
     return _paths.LIB_SLAK
 
 

@@ -162,35 +162,6 @@ inline void launch_g(unsigned grid, unsigned block, cudaStream_t s, Args&&... ar
     launch_k(G::kernel(), grid, block, s, std::forward<Args>(args)...);
 }
 
-// n int32 words set to 0 (the plans' status words and counters)
-__device__ __forceinline__ void k_zero_body(const unsigned bx_, int* __restrict__ p, int64_t n)
-{
-    const int64_t i = (int64_t)bx_ * kBlock + threadIdx.x;
-    if (i < n) p[i] = 0;
-}
-__global__ void __launch_bounds__(kBlock) k_zero(int* __restrict__ p, int64_t n)
-{
-    griddep_enter();
-    k_zero_body(blockIdx.x, p, n);
-}
-struct k_zero_g {
-    static constexpr int kBounds = 1, kMaxT = kBlock, kMinB = 0;
-    template <class... A> __device__ __forceinline__ void operator()(unsigned bx, const A&... a) const { k_zero_body(bx, a...); }
-    static constexpr auto kernel() { return &k_zero; }
-};
-
-// cudaMemsetAsync to 0 of `bytes` (a multiple of 4), or its grouped form
-inline void zero_async(void* p, size_t bytes, cudaStream_t s)
-{
-    if (g_record) {
-        const int64_t n = (int64_t)(bytes / 4);
-        launch_g<k_zero_g>((unsigned)((n + kBlock - 1) / kBlock > 0 ? (n + kBlock - 1) / kBlock : 1), kBlock, s,
-                           static_cast<int*>(p), n);
-        return;
-    }
-    cudaMemsetAsync(p, 0, bytes, s);
-}
-
 // ---------------------------------------------------------------- float4 ops
 __device__ __forceinline__ float4 f4_add(float4 a, float4 b)
 {

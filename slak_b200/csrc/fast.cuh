@@ -1471,28 +1471,4 @@ struct k_g3_bulk_g {
     static constexpr auto kernel() { return &k_g3_bulk<LAK, STATE>; }
 };
 
-// ---------------------------------------------------------------------------------------------
-// 1 for each edge of a general level without a twin (H holds -1), the input of
-// the scan that gives the edges' boundary ranks to the first fast level
-__device__ __forceinline__ void k_export_bflag_body(const unsigned bx_, int E, const int2* __restrict__ H, int* __restrict__ isb)
-{
-    int e = bx_ * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const int2 h = H[e];
-    isb[e] = (h.x < 0) | (h.y < 0);
-}
-__global__ void k_export_bflag(int E, const int2* __restrict__ H, int* __restrict__ isb)
-{
-    griddep_enter();
-    k_export_bflag_body(blockIdx.x, E, H, isb);
-}
-struct k_export_bflag_g {
-    static constexpr int kBounds = 0, kMaxT = kBlock, kMinB = 0;
-    template <class... A> __device__ __forceinline__ void operator()(unsigned bx, const A&... a) const
-    {
-        k_export_bflag_body(bx, a...);
-    }
-    static constexpr auto kernel() { return &k_export_bflag; }
-};
-
 }  // namespace slak

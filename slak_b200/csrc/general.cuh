@@ -27,6 +27,35 @@
 
 namespace slak {
 
+// n int32 words set to 0 (the plans' status words and counters)
+__device__ __forceinline__ void k_zero_body(const unsigned bx_, int* __restrict__ p, int64_t n)
+{
+    const int64_t i = (int64_t)bx_ * kBlock + threadIdx.x;
+    if (i < n) p[i] = 0;
+}
+__global__ void __launch_bounds__(kBlock) k_zero(int* __restrict__ p, int64_t n)
+{
+    griddep_enter();
+    k_zero_body(blockIdx.x, p, n);
+}
+struct k_zero_g {
+    static constexpr int kBounds = 1, kMaxT = kBlock, kMinB = 0;
+    template <class... A> __device__ __forceinline__ void operator()(unsigned bx, const A&... a) const { k_zero_body(bx, a...); }
+    static constexpr auto kernel() { return &k_zero; }
+};
+
+// cudaMemsetAsync to 0 of `bytes` (a multiple of 4), or its grouped form
+inline void zero_async(void* p, size_t bytes, cudaStream_t s)
+{
+    if (g_record) {
+        const int64_t n = (int64_t)(bytes / 4);
+        launch_g<k_zero_g>((unsigned)((n + kBlock - 1) / kBlock > 0 ? (n + kBlock - 1) / kBlock : 1), kBlock, s,
+                           static_cast<int*>(p), n);
+        return;
+    }
+    cudaMemsetAsync(p, 0, bytes, s);
+}
+
 enum : int { SF_OWNER = 1, SF_BOUT = 2, SF_BIN = 4 };
 
 // polygon levels: corner -> face (validating ptr) and the valences in one pass
@@ -983,6 +1012,30 @@ struct k_vp_lak_g {
         k_vp_lak_body<QUAD>(bx, a...);
     }
     static constexpr auto kernel() { return &k_vp_lak<QUAD>; }
+};
+
+// ---------------------------------------------------------------------------------------------
+// 1 for each edge of a general level without a twin (H holds -1), the input of
+// the scan that gives the edges' boundary ranks to the first fast level
+__device__ __forceinline__ void k_export_bflag_body(const unsigned bx_, int E, const int2* __restrict__ H, int* __restrict__ isb)
+{
+    int e = bx_ * blockDim.x + threadIdx.x;
+    if (e >= E) return;
+    const int2 h = H[e];
+    isb[e] = (h.x < 0) | (h.y < 0);
+}
+__global__ void k_export_bflag(int E, const int2* __restrict__ H, int* __restrict__ isb)
+{
+    griddep_enter();
+    k_export_bflag_body(blockIdx.x, E, H, isb);
+}
+struct k_export_bflag_g {
+    static constexpr int kBounds = 0, kMaxT = kBlock, kMinB = 0;
+    template <class... A> __device__ __forceinline__ void operator()(unsigned bx, const A&... a) const
+    {
+        k_export_bflag_body(bx, a...);
+    }
+    static constexpr auto kernel() { return &k_export_bflag; }
 };
 
 }  // namespace slak

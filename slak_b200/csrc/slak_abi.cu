@@ -21,69 +21,15 @@
 #include <cmath>
 #include <map>
 #include <type_traits>
-#include <cudaTypedefs.h>
 
-#include "common.cuh"
+#include "plan.cuh"
 #include "general.cuh"
-#include "fast.cuh"
-#include "grand.cuh"
 #include "scan.cuh"
 #include "crease.cuh"
 
 using namespace slak;
 
 namespace {
-
-struct Level {
-    int64_t F = 0, V = 0, N = 0, B = 0, E = 0;
-    int64_t Fo = 0, Vo = 0, No = 0;
-    bool quad = true;       // implicit 4-corner faces
-    bool poly_fn = false;   // the reference's first-level (polygon) functions
-    bool fast = false;      // closed-form refinement from the parent level's state
-    bool export_state = false;   // general level whose state feeds a fast level
-    bool make_state = false;     // fast level whose state feeds the next fast level
-    // fast level whose parent's parent is a closed quad mesh (GQ, fast.cuh):
-    // k_g1 sums most of the parent's vertex columns; that mesh's sizes
-    bool gq = false;
-    int64_t gN = 0, gV = 0, gF = 0;
-    // the last GQ level: it takes its parent's state in closed form from the
-    // grandparent's (SG, fast.cuh), so the level before writes none
-    bool sg = false;
-    // closed level with a grandparent (grand.cuh): refined from the
-    // grandparent's state and the parent's quads
-    bool pp = false;
-    bool skip_ids = false;       // its refined quads are read by no later level
-    // k_g3 with bulk-copied slot records (SLAK_PLAN_BULK_RECORDS, closed parents)
-    bool bulk3 = false;
-    int bulk_polls = 0;
-    DevStatus* st = nullptr;
-    QState in_state{}, out_state{};
-    SlotScratch slots{};    // fast level: slot-ordered records from k_g1 to k_g3
-    const int* ptr = nullptr;
-    const int* ids = nullptr;
-    const float* verts = nullptr;
-    int* o_ids = nullptr;
-    float* o_verts = nullptr;
-    int* o_ptr = nullptr;
-    int* o_vals = nullptr;
-    int* scan_tmp = nullptr;       // fast level with a boundary (SLAK, state): scan of C's boundary edges
-    // fast level: block size of k_g1, k_g2, k_g3 (chosen by the autotuner)
-    int bs[3] = {256, 256, 256};
-    int tuned = 0;                 // 0 default, 1 measured now, 2 from the tuning cache
-    float tune_ms[3][3] = {};      // measured ms of each kernel at block 128 / 256 / 512
-    std::string tune_key;
-};
-
-constexpr int kTuneBlocks[3] = {128, 256, 512};
-
-// Calls f with the block size as a compile-time constant.
-template <class F>
-void with_block(int bs, F&& f)
-{
-    if (bs == 128) f(std::integral_constant<int, 128>{});
-    else if (bs == 512) f(std::integral_constant<int, 512>{});
-    else f(std::integral_constant<int, 256>{});
-}
 
 struct Scratch {
     int *cface = nullptr, *cnt = nullptr, *sptr = nullptr, *sc = nullptr, *snext = nullptr, *sprev = nullptr,
@@ -108,59 +54,6 @@ struct Carver {
         T* p = dry ? nullptr : reinterpret_cast<T*>(base + off);
         off += bytes;
         return p;
-    }
-};
-
-// Launch bookkeeping: counts launches and, in debug mode (SLAK_DEBUG_SYNC=1 in
-// the environment when the plan is created), synchronises after every launch
-// and records which kernel failed.
-thread_local std::string g_detail;
-
-struct KernelRec {
-    const char* name;
-    int level;
-    int64_t bytes;
-};
-
-struct Lc {
-    cudaStream_t s;
-    int64_t* nl;
-    bool debug;
-    int level;
-    int err = 0;
-    std::vector<cudaEvent_t>* ev = nullptr;   // timing: one event after every launch (ev[0] before the first)
-    std::vector<KernelRec>* recs = nullptr;
-    // independent kernels of a level on side streams (fork / join by events);
-    // off while timing (per-launch events need one stream) and when debugging
-    bool conc = false;
-    cudaStream_t side[2] = {nullptr, nullptr};
-    cudaEvent_t cev[4] = {nullptr, nullptr, nullptr, nullptr};
-    // side stream k waits for the work enqueued so far on s
-    void fork(int k)
-    {
-        cudaEventRecord(cev[k], s);
-        cudaStreamWaitEvent(side[k], cev[k], 0);
-    }
-    // s waits for side stream k
-    void join(int k)
-    {
-        cudaEventRecord(cev[2 + k], side[k]);
-        cudaStreamWaitEvent(s, cev[2 + k], 0);
-    }
-    void after(const char* name, int n = 1, int64_t bytes = 0)
-    {
-        *nl += n;
-        if (ev && recs->size() + 1 < ev->size()) {
-            cudaEventRecord((*ev)[recs->size() + 1], s);
-            recs->push_back(KernelRec{name, level, bytes});
-        }
-        if (!debug || err) return;
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            err = e == cudaErrorMemoryAllocation ? SLAK_ERR_OOM : SLAK_ERR_CUDA;
-            g_detail = std::string(name) + " (level " + std::to_string(level) + "): " + cudaGetErrorString(e);
-        }
     }
 };
 
@@ -270,6 +163,17 @@ void carve_state(Carver& cv, QState& q, int64_t N, int64_t V, int64_t E)
     q.brank = E ? cv.take<int>(E + 1) : nullptr;
 }
 
+}  // namespace
+
+int slak::scan_launch(const int* in, int* out, int64_t n, int* tmp, cudaStream_t s)
+{
+    int64_t nl = 0;
+    scan_exclusive(in, out, n, tmp, s, &nl);
+    return (int)nl;
+}
+
+namespace {
+
 // Topology of a level up to the edge-offset scan (needs no output buffers).
 void launch_topology_a(const Level& L, int li, int scheme, Scratch& s, DevStatus* st, Lc& lc)
 {
@@ -376,202 +280,6 @@ void launch_rest(const Level& L, int li, int scheme, bool compensated, Scratch& 
     if (lc.conc) { lc.join(0); lc.join(1); }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
-{
-    static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-    });
-    return enc;
-}
-
-// The tensor map of a level's refined quads for k_g1's tensor store: `rows`
-// rows of 16 int32 (thread x's four quads at out + 16 x), boxes of `bs` rows,
-// 64-byte swizzle (the layout k_g1 stages them in).  A null `out` (a launch
-// sequence recorded before any memory exists) leaves the map zeroed.
-bool quad_store_map(CUtensorMap& m, int* out, int64_t rows, int bs)
-{
-    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (out == nullptr) return true;
-    if (enc == nullptr || rows < 1) {
-        g_detail = "cuTensorMapEncodeTiled unavailable";
-        return false;
-    }
-    const cuuint64_t dims[2] = {16, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {64};
-    const cuuint32_t box[2] = {16, (cuuint32_t)bs};
-    const cuuint32_t es[2] = {1, 1};
-    const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, out, dims, strides, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) g_detail = "cuTensorMapEncodeTiled: error " + std::to_string((int)r);
-    return r == CUDA_SUCCESS;
-}
-
-// The same of a PP level (grand.cuh): thread y's 256 bytes as two rows of 128
-// (halves of one row of 64 int32), boxes of one half of `bs` threads, 128-byte
-// swizzle.
-bool quad_store_map2(CUtensorMap& m, int* out, int64_t rows, int bs)
-{
-    if (out == nullptr) return true;
-    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (enc == nullptr || rows < 1) {
-        g_detail = "cuTensorMapEncodeTiled unavailable";
-        return false;
-    }
-    const cuuint64_t dims[3] = {32, 2, (cuuint64_t)rows};
-    const cuuint64_t strides[2] = {128, 256};
-    const cuuint32_t box[3] = {32, 1, (cuuint32_t)bs};
-    const cuuint32_t es[3] = {1, 1, 1};
-    const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, out, dims, strides, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) g_detail = "cuTensorMapEncodeTiled: error " + std::to_string((int)r);
-    return r == CUDA_SUCCESS;
-}
-
-// One fast level: C = L (refined from its parent level Pl, whose state is
-// L.in_state).  BND: Pl has a boundary (quad faces only).
-template <bool LAK, bool STATE, bool PQ, bool BND, bool GQ = false, bool SG = false>
-void launch_fast_t(const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc& lc)
-{
-    FastDims d{(int)Pl.N, (int)Pl.V, (int)Pl.F, (int)Pl.E, (int)L.V, (int)L.N, (int)Pl.B};
-    if (GQ || SG) { d.N2 = (int)L.gN; d.V2 = (int)L.gV; d.F2 = (int)L.gF; }
-    const int nv3 = GQ ? (int)L.gV : (int)Pl.V;      // k_g3's vertices
-    cudaStream_t str = lc.s;
-    // compulsory bytes of each kernel: the level's corner ids and positions it
-    // must read once, and the refined ids / positions it alone writes
-    const int64_t g1b = 4 * L.N + 16 * L.V + (L.skip_ids ? 0 : 16 * L.N) + 16 * L.F + 16 * Pl.F + (LAK ? 0 : 16 * L.F);
-    const int64_t g2b = 16 * Pl.E + (LAK ? 16 * 2 * L.F : 0);
-    // LAK's last level: the refined ptr / vals come from k_g1 too
-    int* optr = LAK && !STATE ? L.o_ptr : nullptr;
-    int4* ovals = LAK && !STATE ? reinterpret_cast<int4*>(L.o_vals) : nullptr;
-    bool mapped = true;
-    with_block(L.bs[0], [&](auto b) {
-        constexpr int BS = decltype(b)::value;
-        CUtensorMap otm;
-        std::memset(&otm, 0, sizeof otm);
-        if constexpr (!STATE && kTmaQuadStore && BS <= 256) mapped = quad_store_map(otm, L.o_ids, Pl.N, BS);
-        if (!mapped) return;            // nothing of the level is launched
-        launch_g<k_g1_g<LAK, STATE, PQ, BS, BND, GQ, SG>>(grid_for(L.F, BS), BS, str, d, pf, L.ids, L.verts, L.in_state,
-                                                          L.out_state, reinterpret_cast<int4*>(L.o_ids), otm, L.o_verts,
-                                                          L.slots, optr, ovals);
-    });
-    if (!mapped) {
-        if (!lc.err) lc.err = SLAK_ERR_CUDA;
-        return;
-    }
-    // GQ: k_g1 also writes the vertex points of P's vertices past V2 (and SLAK their slots' edge points)
-    const int64_t gqb = GQ ? 16 * (Pl.V - L.gV) + (LAK ? 0 : 16 * (L.F - L.gN)) : 0;
-    lc.after("k_g1", 1, (PQ ? g1b + g2b : g1b) + (optr ? 4 * (L.N + 1) + 16 * L.N : 0) + gqb);
-    if (!PQ) {      // with quad faces, k_g1 also does k_gf's and k_g2's work
-        // k_gf, k_g2 and k_g3 read only k_g1's records and the level's inputs and
-        // write disjoint outputs: with side streams they run side by side
-        if (lc.conc) { lc.fork(0); lc.fork(1); }
-        launch_g<k_gf_g<LAK, STATE>>(grid_for(Pl.F), kBlock, lc.conc ? lc.side[0] : str, d, Pl.ptr, L.ids, L.verts, L.out_state, L.o_verts, comp ? 1 : 0);
-        lc.after("k_gf");
-        with_block(L.bs[1], [&](auto b) {
-            constexpr int BS = decltype(b)::value;
-            launch_g<k_g2_g<LAK, STATE, PQ, BS, BND>>(grid_for(L.F, BS), BS, lc.conc ? lc.side[1] : str, d, pf, L.ids, L.verts, L.in_state, L.out_state, L.o_verts);
-        });
-        lc.after("k_g2", 1, g2b);
-    }
-    if (!BND && !SG && L.bulk3) {
-        launch_g<k_g3_bulk_g<LAK, STATE>>(grid_for(nv3 + 1, kBulkBlock), kBulkBlock, str, d, L.verts, L.in_state, L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv3, L.st, L.bulk_polls);
-    } else {
-        with_block(L.bs[2], [&](auto b) {
-            constexpr int BS = decltype(b)::value;
-            launch_g<k_g3_g<LAK, STATE, BS, BND, SG>>(grid_for(nv3 + 1, BS), BS, str, d, L.verts, L.in_state, L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv3, nullptr, 0);
-        });
-    }
-    // compulsory bytes: the vertex points of its vertices, SLAK the edge points of their slots
-    const int64_t ns3 = GQ ? L.gN : L.F;
-    lc.after("k_g3", 1, 16 * (int64_t)nv3 + (LAK ? 0 : 16 * ns3));
-    if (BND && STATE && !LAK) {    // C's edges 0..N1-1 (P's slots): boundary ranks by a scan
-        int64_t nl = 0;
-        scan_exclusive(L.slots.bscan, L.out_state.brank, Pl.N, L.scan_tmp, str, &nl);
-        lc.after("scan(boundary)", (int)nl);
-    }
-    if (!PQ && lc.conc) { lc.join(0); lc.join(1); }
-}
-
-template <bool PQ, bool BND, bool GQ = false>
-void launch_fast_p(const Level& Pl, const Level& L, Faces<PQ> pf, bool lak, bool comp, Lc& lc)
-{
-    if constexpr (GQ) {
-        if (L.sg) {             // the last level: no state to write
-            if (lak) launch_fast_t<true, false, PQ, BND, GQ, true>(Pl, L, pf, comp, lc);
-            else launch_fast_t<false, false, PQ, BND, GQ, true>(Pl, L, pf, comp, lc);
-            return;
-        }
-    }
-    if (lak) {
-        if (L.make_state) launch_fast_t<true, true, PQ, BND, GQ>(Pl, L, pf, comp, lc);
-        else launch_fast_t<true, false, PQ, BND, GQ>(Pl, L, pf, comp, lc);
-    } else {
-        if (L.make_state) launch_fast_t<false, true, PQ, BND, GQ>(Pl, L, pf, comp, lc);
-        else launch_fast_t<false, false, PQ, BND, GQ>(Pl, L, pf, comp, lc);
-    }
-}
-
-// One PP level (grand.cuh): C = L, its parent Pl and its parent's parent PPl,
-// whose state is L.in_state.  The block size bs[0] counts C's quads: four per
-// thread of k_pp.
-template <bool LAK, bool STATE, bool PQ>
-void launch_pp_t(const Level& PPl, const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc& lc)
-{
-    FastDims d{(int)Pl.N, (int)Pl.V, (int)Pl.F, (int)Pl.E, (int)L.V, (int)L.N, 0};
-    d.N2 = (int)PPl.N; d.V2 = (int)PPl.V; d.F2 = (int)PPl.F;
-    int* optr = LAK && !STATE ? L.o_ptr : nullptr;
-    int4* ovals = LAK && !STATE ? reinterpret_cast<int4*>(L.o_vals) : nullptr;
-    const int wids = L.skip_ids ? 0 : 1;
-    bool mapped = true;
-    with_block(L.bs[0], [&](auto b) {
-        constexpr int BS = decltype(b)::value / 4;
-        CUtensorMap otm;
-        std::memset(&otm, 0, sizeof otm);
-        if (wids) mapped = quad_store_map2(otm, L.o_ids, PPl.N, BS);
-        if (!mapped) return;            // nothing of the level is launched
-        launch_g<k_pp_g<LAK, STATE, PQ, BS>>(grid_for(PPl.N, BS), BS, lc.s, d, pf, reinterpret_cast<const int4*>(Pl.ids),
-                                             L.verts, L.in_state, L.out_state, wids, otm, L.o_verts, L.slots, optr,
-                                             ovals, comp ? 1 : 0);
-    });
-    if (!mapped) {
-        if (!lc.err) lc.err = SLAK_ERR_CUDA;
-        return;
-    }
-    // compulsory bytes: the parent's quads and C's positions in; the refined
-    // quads, all refined positions but k_g3's out
-    const int64_t g3 = 16 * PPl.V + (LAK ? 0 : 16 * PPl.N);
-    lc.after("k_pp", 1, 16 * PPl.N + 16 * L.V + (wids ? 16 * L.N : 0) + 16 * L.Vo - g3 +
-                            (optr ? 4 * (L.N + 1) + 16 * L.N : 0));
-    const int nv = (int)(PQ ? PPl.V : PPl.V + PPl.F);
-    with_block(L.bs[2], [&](auto b) {
-        constexpr int BS = decltype(b)::value;
-        launch_g<k_g3_g<LAK, STATE, BS, false, false, true>>(grid_for(nv + 1, BS), BS, lc.s, d, L.verts, L.in_state,
-                                                             L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv,
-                                                             PQ ? nullptr : PPl.ptr, kPpFace);
-    });
-    lc.after("k_g3", 1, g3);
-}
-
-template <bool PQ>
-void launch_pp(const Level& PPl, const Level& Pl, const Level& L, Faces<PQ> pf, bool lak, bool comp, Lc& lc)
-{
-    if (lak) {
-        if (L.make_state) launch_pp_t<true, true, PQ>(PPl, Pl, L, pf, comp, lc);
-        else launch_pp_t<true, false, PQ>(PPl, Pl, L, pf, comp, lc);
-    } else {
-        if (L.make_state) launch_pp_t<false, true, PQ>(PPl, Pl, L, pf, comp, lc);
-        else launch_pp_t<false, false, PQ>(PPl, Pl, L, pf, comp, lc);
-    }
-}
-
 // `L` is the level, L[-1] its parent; `cface` is level 0's corner -> face map
 // when it has polygon faces
 void launch_fast(const Level* Lp, const int* cface, int scheme, bool comp, Lc& lc)
@@ -580,15 +288,15 @@ void launch_fast(const Level* Lp, const int* cface, int scheme, bool comp, Lc& l
     const bool lak = scheme == SLAK_SCHEME_LAK;
     if (L.pp) {
         const Level& PPl = Lp[-2];
-        if (PPl.quad) launch_pp<true>(PPl, Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
-        else launch_pp<false>(PPl, Pl, L, Faces<false>{PPl.ptr, cface}, lak, comp, lc);
+        if (PPl.quad) launch_pp_quad(PPl, Pl, L, lak, comp, lc);
+        else launch_pp_poly(PPl, Pl, L, cface, lak, comp, lc);
         return;
     }
-    if (L.gq) launch_fast_p<true, false, true>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
-    else if (Pl.quad && Pl.B > 0) launch_fast_p<true, true>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
-    else if (Pl.quad) launch_fast_p<true, false>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
-    else if (Pl.B > 0) launch_fast_p<false, true>(Pl, L, Faces<false>{Pl.ptr, cface}, lak, comp, lc);
-    else launch_fast_p<false, false>(Pl, L, Faces<false>{Pl.ptr, cface}, lak, comp, lc);
+    if (L.gq) launch_fast_gq(Pl, L, lak, comp, lc);
+    else if (Pl.quad && Pl.B > 0) launch_fast_quad_open(Pl, L, lak, comp, lc);
+    else if (Pl.quad) launch_fast_quad(Pl, L, lak, comp, lc);
+    else if (Pl.B > 0) launch_fast_poly_open(Pl, L, cface, lak, comp, lc);
+    else launch_fast_poly(Pl, L, cface, lak, comp, lc);
 }
 
 // The crease pass of level li (after the level's own kernels): level 0 first
