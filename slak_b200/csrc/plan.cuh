@@ -17,6 +17,8 @@ struct Level {
     bool quad = true;       // implicit 4-corner faces
     bool poly_fn = false;   // the reference's first-level (polygon) functions
     bool fast = false;      // closed-form refinement from the parent level's state
+    bool closed0 = false;        // general level 0 of a closed mesh (closed0.cuh)
+    bool cap0 = false;           // ... none of whose vertices is above valence kC0Cap
     bool export_state = false;   // general level whose state feeds a fast level
     bool make_state = false;     // fast level whose state feeds the next fast level
     // fast level whose parent's parent is a closed quad mesh (GQ, fast.cuh):

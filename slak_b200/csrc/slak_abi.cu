@@ -25,6 +25,7 @@
 #include "plan.cuh"
 #include "general.cuh"
 #include "scan.cuh"
+#include "closed0.cuh"
 #include "crease.cuh"
 
 using namespace slak;
@@ -38,6 +39,11 @@ struct Scratch {
     int2* H = nullptr;
     int *xslot = nullptr, *xtw = nullptr, *xt = nullptr;   // state export of a general quad level
     int *xbrank = nullptr, *xisb = nullptr;                // ... with a boundary: edges' boundary ranks
+    // closed level 0 (closed0.cuh): both counts per vertex, their tile sums, the
+    // corners' ranks and records
+    u64 *cnt2 = nullptr, *tmp2 = nullptr;
+    int* rank = nullptr;
+    int4* rec = nullptr;
 };
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -142,6 +148,29 @@ void carve_scratch(Carver& cv, Scratch& s, int64_t N, int64_t V, int64_t E, bool
     s.eptr = cv.take<int>(V + 1);
     s.tmp = cv.take<int>(scan_tiles(N > V ? N : V) + 2);
     s.H = cv.take<int2>(E);
+}
+
+// scratch of a closed level 0: `cap` no vertex above valence kC0Cap, `slots`
+// the slot-ordered columns are wanted (long columns, creases)
+void carve_closed0(Carver& cv, Scratch& s, int64_t N, int64_t V, bool poly, bool cap, bool slots)
+{
+    s.cnt2 = cv.take<u64>(V);
+    s.tmp2 = cv.take<u64>(scan_tiles(V) + 1);
+    s.cface = poly ? cv.take<int>(N) : nullptr;
+    s.sptr = cv.take<int>(V + 1);
+    s.eptr = cv.take<int>(V + 1);
+    s.rank = cap ? nullptr : cv.take<int>(N);
+    s.rec = cv.take<int4>(cap ? kC0Cap * V : N);
+    s.eid = cv.take<int>(N);
+    s.xslot = cv.take<int>(N);
+    s.xtw = cv.take<int>(N);
+    s.xt = cv.take<int>(N);
+    s.sc = slots ? cv.take<int>(N) : nullptr;
+    s.snext = slots ? cv.take<int>(N) : nullptr;
+    s.sprev = slots ? cv.take<int>(N) : nullptr;
+    s.sprevc = slots ? cv.take<int>(N) : nullptr;
+    s.sflag = slots ? cv.take<int>(N) : nullptr;
+    s.tmp = slots ? cv.take<int>(scan_tiles(V) + 2) : nullptr;      // the creases' scan
 }
 
 // E > 0: the exported level has a boundary, so its edges' boundary ranks go too
@@ -299,6 +328,61 @@ void launch_fast(const Level* Lp, const int* cface, int scheme, bool comp, Lc& l
     else launch_fast_poly(Pl, L, cface, lak, comp, lc);
 }
 
+// A closed level 0 (closed0.cuh); its counts s.cnt2 are zero.
+template <bool QUAD, bool LAK, bool CAP>
+void launch_closed0_t(const Level& L, bool creased, bool comp, Scratch& s, DevStatus* st, Lc& lc)
+{
+    const int F = (int)L.F, V = (int)L.V, N = (int)L.N, E = (int)L.E;
+    cudaStream_t str = lc.s;
+    Faces<QUAD> fc{L.ptr, s.cface};
+    float* R = L.o_verts;
+    float* FPo = R + 4 * (size_t)V;
+    float* EPo = R + 4 * ((size_t)V + (size_t)F);
+    launch_g<k_c0_faces_g<QUAD, LAK, CAP>>(grid_for(F), kBlock, str, L.ptr, L.ids, F, N, V, L.verts, FPo, s.cface, s.cnt2,
+                                           s.rank, s.rec, st);
+    lc.after("k_c0_faces");
+    const int nt = (int)std::max<int64_t>(1, scan_tiles(V));
+    if (nt <= kC0Direct) {
+        launch_g<k_c0_offsets_g<true>>((unsigned)nt, kBlock, str, s.cnt2, V, s.tmp2, nt, s.sptr, s.eptr, N, E, st);
+        lc.after("k_c0_offsets");
+    } else {
+        launch_g<k_c0_sums_g>((unsigned)nt, kBlock, str, s.cnt2, V, s.tmp2);
+        lc.after("k_c0_sums");
+        launch_g<k_c0_offsets_g<false>>((unsigned)nt, kBlock, str, s.cnt2, V, s.tmp2, nt, s.sptr, s.eptr, N, E, st);
+        lc.after("k_c0_offsets");
+    }
+    if (!CAP) {
+        launch_g<k_c0_bucket_g<QUAD>>(grid_for(N), kBlock, str, fc, L.ids, N, F, V, s.sptr, s.rank, s.rec);
+        lc.after("k_c0_bucket");
+    }
+    const C0Out o{s.xslot, s.xtw, s.eid, s.sc, s.snext, s.sprev, s.sprevc, s.sflag, creased ? 1 : 0};
+    launch_g<k_c0_verts_g<QUAD, LAK, CAP>>(grid_for(V, 128), 128, str, L.ptr, V, E, s.sptr, s.eptr, s.rec, o, L.verts,
+                                           FPo, R, comp ? 1 : 0, st);
+    lc.after("k_c0_verts");
+    if (!CAP) {
+        launch_g<k_c0_long_g<QUAD, LAK>>(grid_for(V), kBlock, str, fc, V, E, s.sptr, s.eptr, s.sc, s.snext, s.sprev,
+                                         s.sprevc, s.xtw, s.eid, L.verts, FPo, R, comp ? 1 : 0, st);
+        lc.after("k_c0_long");
+    }
+    launch_g<k_c0_quads_g<QUAD, LAK>>(grid_for(N), kBlock, str, fc, L.ids, s.eid, s.xslot, s.xtw,
+                                      !LAK && L.export_state ? s.xt : nullptr, N, V, F, E,
+                                      reinterpret_cast<int4*>(L.o_ids), L.o_ptr, reinterpret_cast<int4*>(L.o_vals),
+                                      L.verts, FPo, EPo);
+    lc.after("k_c0_quads");
+}
+
+template <bool QUAD>
+void launch_closed0(const Level& L, int scheme, bool creased, bool comp, Scratch& s, DevStatus* st, Lc& lc)
+{
+    if (scheme == SLAK_SCHEME_LAK) {
+        if (L.cap0) launch_closed0_t<QUAD, true, true>(L, creased, comp, s, st, lc);
+        else launch_closed0_t<QUAD, true, false>(L, creased, comp, s, st, lc);
+    } else {
+        if (L.cap0) launch_closed0_t<QUAD, false, true>(L, creased, comp, s, st, lc);
+        else launch_closed0_t<QUAD, false, false>(L, creased, comp, s, st, lc);
+    }
+}
+
 // The crease pass of level li (after the level's own kernels): level 0 first
 // resolves the crease pairs on its vertex columns and lists each base
 // vertex's crease edges.
@@ -368,7 +452,15 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
         lc.recs = &p->recs;
         cudaEventRecord(p->ev[0], str);
     }
-    zero_async(p->st, sizeof(DevStatus), str);
+    // a closed level 0's counts follow the status word in a plan's own arena
+    const bool c0 = !p->lv.empty() && p->lv[0].closed0;
+    const size_t stb = align_up(sizeof(DevStatus)), cnb = c0 ? sizeof(u64) * (size_t)p->lv[0].V : 0;
+    if (c0 && reinterpret_cast<char*>(p->s.cnt2) == reinterpret_cast<char*>(p->st) + stb) {
+        zero_async(p->st, stb + cnb, str);
+    } else {
+        zero_async(p->st, sizeof(DevStatus), str);
+        if (c0) zero_async(p->s.cnt2, cnb, str);
+    }
     const bool comp = (p->flags & SLAK_PLAN_COMPENSATED) != 0;
     for (size_t li = 0; li < p->lv.size(); ++li) {
         const Level& L = p->lv[li];
@@ -376,6 +468,13 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
         if (L.fast) {
             launch_fast(&L, p->s.cface, p->scheme, comp, lc);
             if (lc.err) break;          // a level that could not be launched stops the plan
+            if ((int)li < p->crease_levels) launch_creases(p, (int)li, lc);
+            continue;
+        }
+        if (L.closed0) {
+            const bool creased = p->crease_levels > 0;
+            if (L.quad) launch_closed0<true>(L, p->scheme, creased, comp, p->s, p->st, lc);
+            else launch_closed0<false>(L, p->scheme, creased, comp, p->s, p->st, lc);
             if ((int)li < p->crease_levels) launch_creases(p, (int)li, lc);
             continue;
         }
@@ -534,7 +633,12 @@ int plan_levels(slak_plan* p)
                 L.gN = p->lv[i - 2].N; L.gV = p->lv[i - 2].V; L.gF = p->lv[i - 2].F;
             }
         }
-        if (!L.fast) {
+        if (i == 0 && L.B == 0 && !force_general) {
+            L.closed0 = true;
+            L.cap0 = true;              // no vertex above valence kC0Cap
+            for (int k = kC0Cap + 1; k < 17; ++k) L.cap0 = L.cap0 && p->vhist[k] == 0;
+        }
+        if (!L.fast && !L.closed0) {
             if (L.N > p->maxN) p->maxN = L.N;
             if (L.V > p->maxV) p->maxV = L.V;
             if (L.E > p->maxE) p->maxE = L.E;
@@ -574,8 +678,14 @@ int plan_levels(slak_plan* p)
 void plan_carve(slak_plan* p, Carver& cv)
 {
     const int nlev = (int)p->lv.size();
-    carve_scratch(cv, p->s, p->maxN, p->maxV, p->maxE, p->any_poly);
-    if (p->exN) carve_export(cv, p->s, p->exN, p->exE);
+    p->st = cv.take<DevStatus>(1);
+    if (nlev && p->lv[0].closed0) {
+        const Level& L0 = p->lv[0];
+        carve_closed0(cv, p->s, L0.N, L0.V, !L0.quad, L0.cap0, !L0.cap0 || p->crease_levels > 0);
+    } else {
+        carve_scratch(cv, p->s, p->maxN, p->maxV, p->maxE, p->any_poly);
+        if (p->exN) carve_export(cv, p->s, p->exN, p->exE);
+    }
     p->qs.assign(nlev, QState{});
     for (int i = 0; i < nlev; ++i) {
         const Level& L = p->lv[i];
@@ -597,7 +707,6 @@ void plan_carve(slak_plan* p, Carver& cv)
         if (!p->lv[i].skip_ids) p->mid_ids[i] = cv.take<int>(p->lv[i].No);
         p->mid_verts[i] = cv.take<float>(4 * p->lv[i].Vo);
     }
-    p->st = cv.take<DevStatus>(1);
     if (p->crease_levels > 0) {
         const int64_t m = p->ncrease;
         p->c_pairs = cv.take<int>(2 * m);
