@@ -482,24 +482,25 @@ __device__ __forceinline__ void k_c0_verts_body(const unsigned bx_, const int* _
     }
     if constexpr (!CAP) {
         // longer columns by their warp: slots by rank, twins by search; k_c0_long does the rest
-        unsigned big = __ballot_sync(0xffffffffu, v < V && n > 8);
-        while (big) {
-            const int src = __ffs(big) - 1;
-            big &= big - 1;
-            const int bv = __shfl_sync(0xffffffffu, v, src), bb = __shfl_sync(0xffffffffu, b, src);
-            const int bn = __shfl_sync(0xffffffffu, n, src);
+        for_each_big<128>(v < V && n > 8, true, [&](int i) {
+            const int bv = bx_ * blockDim.x + i, bb = __ldg(sptr + bv), bn = __ldg(sptr + bv + 1) - bb;
             int bad = 0;
             for (int k = lane; k < bn; k += 32) {
                 const int4 me = __ldg(rec + bb + k);
                 const int w = me.y & 0x7fffffff;
-                int tw = -1, rk = 0;
+                int4 hit = make_int4(-1, 0, 0, 0);       // the record entered from w
+                int rk = 0;
 #pragma unroll 8
                 for (int t = 0; t < bn; ++t) {
                     const int4 x = __ldg(rec + bb + t);
                     rk += x.x < me.x;
-                    if (x.z == w) { if (tw < 0) tw = rec_prev<QUAD>(ptr, x); else bad = 1; }
+                    if (x.z == w) {
+                        if (hit.x < 0) hit = x;
+                        else bad = 1;
+                    }
                     if (t < k && (x.y & 0x7fffffff) == w) bad = 1;
                 }
+                const int tw = hit.x < 0 ? -1 : rec_prev<QUAD>(ptr, hit);
                 if (w == bv || me.z == bv || tw < 0) bad = 1;
                 const int s = bb + rk;
                 o.xslot[me.x] = s;
@@ -511,7 +512,7 @@ __device__ __forceinline__ void k_c0_verts_body(const unsigned bx_, const int* _
                 o.sflag[s] = 0;
             }
             if (bad) set_error(st, 4, bv);
-        }
+        });
     }
 }
 template <bool QUAD, bool LAK, bool CAP>
@@ -548,14 +549,11 @@ __device__ __forceinline__ void k_c0_long_body(const unsigned bx_, Faces<QUAD> f
 {
     const int v = bx_ * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    int b = 0, n = 0, id0 = 0;
-    if (v < V) { b = __ldg(sptr + v); n = __ldg(sptr + v + 1) - b; id0 = __ldg(eptr + v); }
-    unsigned m = __ballot_sync(0xffffffffu, v < V && n > 8);
-    while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1;
-        const int bv = __shfl_sync(0xffffffffu, v, src), bb = __shfl_sync(0xffffffffu, b, src);
-        const int bn = __shfl_sync(0xffffffffu, n, src), bid = __shfl_sync(0xffffffffu, id0, src);
+    int b = 0, n = 0;
+    if (v < V) { b = __ldg(sptr + v); n = __ldg(sptr + v + 1) - b; }
+    for_each_big<kBlock>(v < V && n > 8, true, [&](int i) {
+        const int bv = bx_ * blockDim.x + i, bb = __ldg(sptr + bv), bn = __ldg(sptr + bv + 1) - bb;
+        const int bid = __ldg(eptr + bv);
         int before = 0, bad = 0;
         for (int k0 = 0; k0 < bn; k0 += 32) {
             const int k = k0 + lane;
@@ -564,8 +562,10 @@ __device__ __forceinline__ void k_c0_long_body(const unsigned bx_, Faces<QUAD> f
             int rk;
             if (LAK) {
                 rk = 0;
-                if (own)
+                if (own) {
+#pragma unroll 8
                     for (int t = 0; t < bn; ++t) rk += __ldg(snext + bb + t) < w;
+                }
             } else {
                 const unsigned g = __ballot_sync(0xffffffffu, own);
                 rk = before + __popc(g & ((1u << lane) - 1));
@@ -586,7 +586,7 @@ __device__ __forceinline__ void k_c0_long_body(const unsigned bx_, Faces<QUAD> f
             else
                 vp_slak_warp<QUAD>(fc, sc, snext, sprev, nullptr, 0, P, FP, R, compensated, bv, bb, bn);
         }
-    }
+    });
     if (v < V && n > 8 && (n <= kBigCol || n > kWarpCol)) {
         if constexpr (LAK)
             vp_lak_vertex<QUAD>(fc, sc, snext, sprev, sprevc, nullptr, eid, 0, P, FP, R, compensated, v, b, n);

@@ -286,31 +286,113 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src)
                        __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
 }
 
-// A long column's slots in its warp: slot k is element k >> 5 of lane k & 31
-// (two per lane for up to kWarpCol = 64 slots).  col4 / col1 fetch slot k
-// (k the same on every lane) from its lane; rank_of gives each of a lane's
-// keys its rank in ascending key order, ties by slot.
-__device__ __forceinline__ float4 col4(float4 e0, float4 e1, int k) { return shfl4(k < 32 ? e0 : e1, k & 31); }
+// A long column's keys in its warp: slot k is element k >> 5 of lane k & 31
+// (two per lane for up to kWarpCol = 64 slots).  col1 fetches slot k (k the
+// same on every lane) from its lane; column_order gives the slots in ascending
+// key order, ties by slot: order[rank] = slot, in the warp's row of shared
+// memory.
 __device__ __forceinline__ int col1(int e0, int e1, int k) { return __shfl_sync(0xffffffffu, k < 32 ? e0 : e1, k & 31); }
-__device__ __forceinline__ void rank_of(int n, int key0, int key1, int& r0, int& r1)
+__device__ __forceinline__ void column_order(int n, int key0, int key1, unsigned char* order)
 {
     const int lane = threadIdx.x & 31;
-    r0 = 0;
-    r1 = 0;
+    int r0 = 0, r1 = 0;
+#pragma unroll 8
     for (int j = 0; j < n; ++j) {
         const int y = col1(key0, key1, j);
         r0 += (y < key0) | ((y == key0) & (j < lane));
         r1 += (y < key1) | ((y == key1) & (j < lane + 32));
     }
+    if (lane < n) order[r0] = (unsigned char)lane;
+    if (lane + 32 < n) order[r1] = (unsigned char)(lane + 32);
+    __syncwarp();
 }
-// The slot of rank r (r the same on every lane), as (lane, element).
-__device__ __forceinline__ void slot_of_rank(int r, bool h0, bool h1, int r0, int r1, int& src, int& el)
+// A long column's terms, one component per lane: lane l holds component l & 3
+// of terms 8j + (l >> 2), j = 0..7, so a step of a sum in column order is one
+// shuffle and one scalar add (as float4, two slots per lane, it was four
+// shuffles and all four components' adds on every lane).  Such a column is a
+// serial chain beside which the level waits: with two 64-slot poles and
+// compensated sums (capped cylinder, B200), this, all of a column's loads in
+// flight at once and for_each_big took k_g3 of its small levels from 18.4 to
+// 14.3 us each (8 us without poles), k_c0_verts from 38 to 15 and k_c0_long from
+// 19 to 12 us.
+__device__ __forceinline__ int term_slot() { return (threadIdx.x & 31) >> 2; }
+__device__ __forceinline__ int term_comp() { return threadIdx.x & 3; }
+template <class Add>
+__device__ __forceinline__ void each_term(const float (&x)[8], int n, Add add)
 {
-    const unsigned m0 = __ballot_sync(0xffffffffu, h0 && r0 == r);
-    const unsigned m1 = __ballot_sync(0xffffffffu, h1 && r1 == r);
-    el = m0 ? 0 : 1;
-    src = __ffs(m0 ? m0 : m1) - 1;
+    const int c = term_comp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (8 * j >= n) break;
+        const int m = n - 8 * j < 8 ? n - 8 * j : 8;
+        float t = __shfl_sync(0xffffffffu, x[j], c);
+#pragma unroll 1
+        for (int i = 1; i <= m; ++i) {          // the next term on its way while this one is added
+            const float tn = __shfl_sync(0xffffffffu, x[j], ((4 * i) & 31) + c);
+            add(t);
+            t = tn;
+        }
+    }
 }
+// f(i) by a whole warp for each thread i of the block with `big` set.  SPREAD:
+// over the block's warps (the two poles of a sphere are often neighbours, and
+// a column's serial sum is microseconds); else by the thread's own warp, without
+// a barrier.  Every thread of the block takes part, `spread` the same on all.
+template <int BS, class F>
+__device__ __forceinline__ void for_each_big(bool big, bool spread, F f)
+{
+    __shared__ unsigned short list[BS];
+    __shared__ int count;
+    if (!spread) {
+        unsigned m = __ballot_sync(0xffffffffu, big);
+        while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1;
+            f((int)(threadIdx.x & ~31u) + src);
+        }
+        return;
+    }
+    if (!__syncthreads_or(big)) return;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    if (big) list[atomicAdd(&count, 1)] = (unsigned short)threadIdx.x;
+    __syncthreads();
+    for (int i = threadIdx.x >> 5; i < count; i += BS / 32) f((int)list[i]);
+}
+__device__ __forceinline__ float div1(float a, float s)
+{
+    float r;
+    return pow2_recip(s, r) ? __fmul_rn(a, r) : __fdiv_rn(a, s);
+}
+// The vertex point of a column of n slots from its neighbours (SLAK: slot
+// order; LAK: ascending id) and face points (slot order); p: component l & 3 of
+// the vertex.  Every lane returns the whole point.
+template <bool LAK>
+__device__ __forceinline__ float4 column_point(const float (&nb)[8], const float (&fp)[8], float p, int n, bool comp)
+{
+    const float nn = (float)(n * n), fn = (float)n;
+    float acc = 0.0f, lo = 0.0f, y;
+    const auto sum = [&](float t) { acc = __fadd_rn(acc, t); };
+    const auto dd = [&](float t) { dd_acc1(acc, lo, t); };
+    if (comp) {
+        if (LAK) { each_term(fp, n, dd); each_term(nb, n, dd); }
+        else { each_term(nb, n, dd); each_term(fp, n, dd); }
+        y = vp_finish1(acc, lo, p, n);
+    } else if (!LAK) {
+        each_term(nb, n, sum);
+        y = __fadd_rn(div1(acc, nn), div1(__fmul_rn(p, (float)(n - 2)), fn));
+        each_term(fp, n, [&](float t) { y = __fadd_rn(y, div1(t, nn)); });
+    } else {
+        each_term(fp, n, sum);
+        each_term(nb, n, sum);
+        const float m = __fadd_rn(div1(acc, fn), 0.0f);
+        y = __fadd_rn(div1(__fadd_rn(m, __fmul_rn(p, __fadd_rn(fn, -2.0f))), fn), 0.0f);
+    }
+    return make_float4(__shfl_sync(0xffffffffu, y, 0), __shfl_sync(0xffffffffu, y, 1), __shfl_sync(0xffffffffu, y, 2),
+                       __shfl_sync(0xffffffffu, y, 3));
+}
+__device__ __forceinline__ float ldg1(const float* p, int64_t i, int c) { return __ldg(p + 4 * i + c); }
+
 // The slots k = 0..n-1 of key[b..b+n) in ascending key order (equal keys by
 // slot): perm[r] = the slot of rank r.  n^2 independent compares, instead of
 // n selection passes that each wait for the previous minimum; for one thread's

@@ -1221,78 +1221,57 @@ __device__ __forceinline__ void g3_vertex(FastDims d, const float* __restrict__ 
 }
 
 // A long column (kBigCol < n <= kWarpCol; the poles of high-valence meshes),
-// by the whole warp: each lane loads its (up to two) slots' records, LAK tails
-// are ranked by id across the warp, SLAK's edge points are independent per
-// slot; the sums run in the order the single-thread path uses, every lane
-// fetching slot k (or the tail of rank r) by shuffle, so the result is the
-// same bit for bit.  No shared memory: the common path keeps its L1.
+// by the whole warp: LAK tails are ranked by id across the warp, SLAK's edge
+// points are independent per slot; the sums run in the order the single-thread
+// path uses, one component per lane (column_point), so the result is the same
+// bit for bit.
 template <bool LAK, bool STATE, bool BND, bool PP = false>
 __device__ __noinline__ void g3_warp_column(FastDims d, const float* __restrict__ P, QState c, SlotScratch z,
                                             float* __restrict__ R, int compensated, int v, int b, int n)
 {
-    const int lane = threadIdx.x & 31;
+    __shared__ unsigned char order[LAK ? 16 : 1][LAK ? kWarpCol : 1];
+    const int lane = threadIdx.x & 31, c4 = term_comp();
     const float4* Z = z.Z;
-    const bool h0 = lane < n, h1 = lane + 32 < n;
-    const int k0 = b + lane, k1 = b + lane + 32;
-    float4 f0 = f4_zero(), f1 = f4_zero(), n0 = f4_zero(), n1 = f4_zero();   // FP(x) and the neighbour
-    int t0 = INT32_MAX, t1 = INT32_MAX;
-    // two 16-byte loads per record here: ptxas 12.9 fails on the 256-bit load in this function
-    if (h0) { f0 = rec_f<LAK, PP>(Z, k0); n0 = rec_n<LAK, PP>(d, P, Z, k0); if (LAK) t0 = __ldg(z.T + k0); }
-    if (h1) { f1 = rec_f<LAK, PP>(Z, k1); n1 = rec_n<LAK, PP>(d, P, Z, k1); if (LAK) t1 = __ldg(z.T + k1); }
     const float4 Pv = ldg4(P, v);
-    if (!LAK) {
-        // edge points of C's edges {v, e_out(x)}, ids b..e-1: 0 + (p_v + FP(x))/4 + (Z[2s+1] + Z[2 rot[s]])/4,
-        // FP of slot rot[s] from the lane that holds it
-        const int64_t EPb = (int64_t)d.V + d.N1;
+    unsigned char* ord = order[LAK ? threadIdx.x >> 5 : 0];
+    if constexpr (LAK)             // the tails in ascending id
+        column_order(n, lane < n ? __ldg(z.T + b + lane) : INT32_MAX, lane + 32 < n ? __ldg(z.T + b + lane + 32) : INT32_MAX,
+                     ord);
+    const float pv = c4 == 0 ? Pv.x : c4 == 1 ? Pv.y : c4 == 2 ? Pv.z : Pv.w;
+    float nb[8], fp[8], fr[8];
+    const float* Zf = reinterpret_cast<const float*>(Z);
 #pragma unroll
-        for (int el = 0; el < 2; ++el) {
-            const bool h = el ? h1 : h0;
-            const int k = el ? k1 : k0;
-            const int q = h ? __ldg(z.rot + k) - b : 0;
-            const float4 a = shfl4(f0, q & 31), a1 = shfl4(f1, q & 31);
-            if (!h) continue;
-            const float4 fr = q < 32 ? a : a1, nk = el ? n1 : n0, fk = el ? f1 : f0;
-            if (BND && (__ldg(z.bflag + k) & 1)) {
-                st4_cs(R, EPb + k, f4_mul(f4_add(Pv, nk), 0.5f));
-                continue;
+    for (int j = 0; j < 8; ++j) {
+        const int k = 8 * j + term_slot();
+        nb[j] = fp[j] = fr[j] = 0.0f;
+        if (k < n) {
+            if constexpr (PP && !LAK) {
+                nb[j] = ldg1(P, (int64_t)d.V1 + d.F1 + b + k, c4);
+                fp[j] = ldg1(Zf, (int64_t)b + k, c4);
+                fr[j] = ldg1(Zf, __ldg(z.rot + b + k), c4);
+            } else {
+                nb[j] = ldg1(Zf, 2 * (int64_t)(b + (LAK ? ord[k] : k)) + 1, c4);
+                fp[j] = ldg1(Zf, 2 * (int64_t)(b + k), c4);
+                if (!LAK) fr[j] = ldg1(Zf, 2 * (int64_t)__ldg(z.rot + b + k), c4);
             }
-            const float4 ta = f4_mul(f4_add(Pv, fk), 0.25f);
-            st4_cs(R, EPb + k, f4_add(f4_add(f4_zero(), ta), f4_mul(f4_add(nk, fr), 0.25f)));
         }
     }
-    // every lane runs the sums (the same values, by shuffle); lane 0 stores
-    const bool comp = compensated != 0;
-    const float nn = (float)(n * n);
-    float4 yv;
-    if (!LAK) {
-        if (!comp) {
-            float4 acc = f4_zero();
-            for (int k = 0; k < n; ++k) acc = f4_add(acc, col4(n0, n1, k));
-            yv = f4_add(f4_div(acc, nn), f4_div(f4_mul(Pv, (float)(n - 2)), (float)n));
-            for (int k = 0; k < n; ++k) yv = f4_add(yv, f4_div(col4(f0, f1, k), nn));
-        } else {
-            float4 sh = f4_zero(), sl = f4_zero();
-            for (int k = 0; k < n; ++k) dd_acc(sh, sl, col4(n0, n1, k));
-            for (int k = 0; k < n; ++k) dd_acc(sh, sl, col4(f0, f1, k));
-            yv = vp_finish(sh, sl, Pv, n);
+    __syncwarp();
+    if constexpr (!LAK) {
+        // edge points of C's edges {v, e_out(x)}, ids b..e-1: 0 + (p_v + FP(x))/4 + (Z[2s+1] + Z[2 rot[s]])/4
+        float* EP = R + 4 * ((int64_t)d.V + d.N1 + b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = 8 * j + term_slot();
+            if (k < n) {
+                float r = __fadd_rn(__fadd_rn(0.0f, __fmul_rn(__fadd_rn(pv, fp[j]), 0.25f)),
+                                    __fmul_rn(__fadd_rn(nb[j], fr[j]), 0.25f));
+                if (BND && (__ldg(z.bflag + b + k) & 1)) r = __fmul_rn(__fadd_rn(pv, nb[j]), 0.5f);
+                __stcs(EP + 4 * k + c4, r);
+            }
         }
-    } else {
-        int r0, r1;
-        rank_of(n, t0, t1, r0, r1);                                  // tails in ascending id
-        float4 acc = f4_zero(), sh = f4_zero(), sl = f4_zero();
-        for (int k = 0; k < n; ++k) {
-            const float4 t = col4(f0, f1, k);
-            if (comp) dd_acc(sh, sl, t); else acc = f4_add(acc, t);
-        }
-        for (int r = 0; r < n; ++r) {
-            int src, el;
-            slot_of_rank(r, h0, h1, r0, r1, src, el);
-            const float4 t = shfl4(el ? n1 : n0, src);
-            if (comp) dd_acc(sh, sl, t); else acc = f4_add(acc, t);
-        }
-        if (comp) yv = vp_finish(sh, sl, Pv, n);
-        else yv = f4_div_z(f4_add(f4_div_z(acc, (float)n), f4_mul(Pv, __fadd_rn((float)n, -2.0f))), (float)n);
     }
+    float4 yv = column_point<LAK>(nb, fp, pv, n, compensated != 0);
     if (lane == 0) {
         if (BND) yv = boundary_vertex<LAK>(P, z, b, b + n, Pv, yv);
         st_pos<STATE>(R, v, yv);
@@ -1310,42 +1289,45 @@ __device__ __noinline__ void g3_warp_column(FastDims d, const float* __restrict_
 // PP's V2 old ones, which keep their columns, then, for a polygon PP (`pptr`
 // its face offsets), the F2 face points, of which the long faces' are summed
 // here.
+// k_g3's `mode`: compensated sums; long columns are expected (spread them over
+// the block's warps)
+enum : int { G3_COMP = 1, G3_LONG = 2 };
 template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false, bool PP = false>
 __device__ __forceinline__ void k_g3_body(const unsigned bx_, FastDims d, const float* __restrict__ P, QState p, QState c,
-                                          SlotScratch z, float* __restrict__ R, int compensated, int nv,
+                                          SlotScratch z, float* __restrict__ R, int mode, int nv,
                                           const int* __restrict__ pptr, int ppface)
 {
-    const int v = bx_ * blockDim.x + threadIdx.x;
+    const int v = bx_ * BS + threadIdx.x;
+    const int comp = mode & G3_COMP;
     if (STATE && v == nv) c.sptr[d.V] = d.N;
-    bool valid = v < nv;
-    int b = 0, n = 0;
-    if (valid) {
+    const auto column = [&](int v, int& b, int& n) {       // false: nothing to sum here
         if constexpr (SG) { b = sg_sptr(d, p.sptr, v); n = sg_sptr(d, p.sptr, v + 1) - b; }
         else if (PP && v >= d.V2) {
             b = __ldg(pptr + v - d.V2);
             n = __ldg(pptr + v - d.V2 + 1) - b;
             b += d.N2;
-            valid = n > ppface;
+            return n > ppface;
         }
         else { b = __ldg(p.sptr + v); n = __ldg(p.sptr + v + 1) - b; }
-    }
+        return true;
+    };
+    int b = 0, n = 0;
+    const bool valid = v < nv && column(v, b, n);
     const bool big = valid && n > kBigCol && n <= kWarpCol;
-    if (valid && !big) g3_vertex<LAK, STATE, BND, PP>(d, P, c, z, R, compensated, v, b, n);
-    unsigned m = __ballot_sync(0xffffffffu, big);
-    while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1;
-        g3_warp_column<LAK, STATE, BND, PP>(d, P, c, z, R, compensated, __shfl_sync(0xffffffffu, v, src),
-                                            __shfl_sync(0xffffffffu, b, src), __shfl_sync(0xffffffffu, n, src));
-    }
+    if (valid && !big) g3_vertex<LAK, STATE, BND, PP>(d, P, c, z, R, comp, v, b, n);
+    for_each_big<BS>(big, mode & G3_LONG, [&](int i) {
+        int bb, bn;
+        column(bx_ * BS + i, bb, bn);
+        g3_warp_column<LAK, STATE, BND, PP>(d, P, c, z, R, comp, bx_ * BS + i, bb, bn);
+    });
 }
 template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false, bool PP = false>
 __global__ void __launch_bounds__(BS) k_g3(FastDims d, const float* __restrict__ P, QState p, QState c,
-                                           SlotScratch z, float* __restrict__ R, int compensated, int nv,
+                                           SlotScratch z, float* __restrict__ R, int mode, int nv,
                                            const int* __restrict__ pptr, int ppface)
 {
     griddep_enter();
-    k_g3_body<LAK, STATE, BS, BND, SG, PP>(blockIdx.x, d, P, p, c, z, R, compensated, nv, pptr, ppface);
+    k_g3_body<LAK, STATE, BS, BND, SG, PP>(blockIdx.x, d, P, p, c, z, R, mode, nv, pptr, ppface);
 }
 template <bool LAK, bool STATE, int BS, bool BND = false, bool SG = false, bool PP = false>
 struct k_g3_g {

@@ -761,9 +761,8 @@ __device__ __forceinline__ void vp_slak_vertex(Faces<QUAD> fc, const int* __rest
     st4(R, v, y);
 }
 
-// a long column (kBigCol < n <= kWarpCol) by its warp: each lane loads its (up
-// to two) slots; the sums run in column order with every lane fetching slot k
-// by shuffle; lane 0 stores
+// a long column (kBigCol < n <= kWarpCol) by its warp, one component per lane
+// (column_point); lane 0 stores
 template <bool QUAD>
 __device__ __noinline__ void vp_slak_warp(Faces<QUAD> fc, const int* __restrict__ sc,
                                           const int* __restrict__ snext, const int* __restrict__ sprev,
@@ -771,23 +770,18 @@ __device__ __noinline__ void vp_slak_warp(Faces<QUAD> fc, const int* __restrict_
                                           const float* __restrict__ FP, float* __restrict__ R, int compensated,
                                           int v, int b, int n)
 {
-    const int lane = threadIdx.x & 31;
-    float4 a0 = f4_zero(), a1 = f4_zero(), f0 = f4_zero(), f1 = f4_zero();    // neighbour, face point
-    if (lane < n) { a0 = ldg4(P, __ldg(snext + b + lane)); f0 = ldg4(FP, fc.face(__ldg(sc + b + lane))); }
-    if (lane + 32 < n) { a1 = ldg4(P, __ldg(snext + b + lane + 32)); f1 = ldg4(FP, fc.face(__ldg(sc + b + lane + 32))); }
-    const float nn = (float)(n * n);
-    float4 y;
-    if (!compensated) {
-        float4 acc = f4_zero();
-        for (int k = 0; k < n; ++k) acc = f4_add(acc, col4(a0, a1, k));
-        y = f4_add(f4_div(acc, nn), f4_div(f4_mul(ldg4(P, v), (float)(n - 2)), (float)n));
-        for (int k = 0; k < n; ++k) y = f4_add(y, f4_div(col4(f0, f1, k), nn));
-    } else {
-        float4 sh = f4_zero(), sl = f4_zero();
-        for (int k = 0; k < n; ++k) dd_acc(sh, sl, col4(a0, a1, k));
-        for (int k = 0; k < n; ++k) dd_acc(sh, sl, col4(f0, f1, k));
-        y = vp_finish(sh, sl, ldg4(P, v), n);
+    const int lane = threadIdx.x & 31, c = term_comp();
+    float nb[8], fp[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int k = 8 * j + term_slot();
+        nb[j] = fp[j] = 0.0f;
+        if (k < n) {
+            nb[j] = ldg1(P, __ldg(snext + b + k), c);
+            fp[j] = ldg1(FP, fc.face(__ldg(sc + b + k)), c);
+        }
     }
+    float4 y = column_point<false>(nb, fp, ldg1(P, v, c), n, compensated != 0);
     if (lane == 0) {
         if (boundary) y = vp_slak_boundary(snext, sprev, sflag, P, v, b, b + n, y);
         st4(R, v, y);
@@ -919,9 +913,9 @@ __device__ __forceinline__ void vp_lak_vertex(Faces<QUAD> fc, const int* __restr
     st4(R, v, y);
 }
 
-// a long column (kBigCol < n <= kWarpCol) by its warp: each lane loads its (up
-// to two) slots, the tails are ranked by id across the warp, and the sums run
-// in the fixed order with every lane fetching by shuffle; lane 0 stores
+// a long column (kBigCol < n <= kWarpCol) by its warp: the tails are ranked by
+// id across the warp, the sums run one component per lane (column_point); lane
+// 0 stores
 template <bool QUAD>
 __device__ __noinline__ void vp_lak_warp(Faces<QUAD> fc, const int* __restrict__ sc,
                                          const int* __restrict__ snext, const int* __restrict__ sprev,
@@ -930,35 +924,24 @@ __device__ __noinline__ void vp_lak_warp(Faces<QUAD> fc, const int* __restrict__
                                          const float* __restrict__ FP, float* __restrict__ R, int compensated,
                                          int v, int b, int n)
 {
-    const int lane = threadIdx.x & 31;
-    const bool h0 = lane < n, h1 = lane + 32 < n;
-    float4 f0 = f4_zero(), f1 = f4_zero(), p0 = f4_zero(), p1 = f4_zero();    // face point, tail position
-    int t0 = INT32_MAX, t1 = INT32_MAX;                                     // tail ids
-    if (h0) { f0 = ldg4(FP, fc.face(__ldg(sc + b + lane))); t0 = __ldg(sprev + b + lane); p0 = ldg4(P, t0); }
-    if (h1) { f1 = ldg4(FP, fc.face(__ldg(sc + b + lane + 32))); t1 = __ldg(sprev + b + lane + 32); p1 = ldg4(P, t1); }
-    int r0, r1;
-    rank_of(n, t0, t1, r0, r1);
-    float4 y;
-    if (!compensated) {
-        float4 acc = f4_zero();
-        for (int k = 0; k < n; ++k) acc = f4_add(acc, col4(f0, f1, k));
-        for (int r = 0; r < n; ++r) {
-            int src, el;
-            slot_of_rank(r, h0, h1, r0, r1, src, el);
-            acc = f4_add(acc, shfl4(el ? p1 : p0, src));
+    __shared__ unsigned char order[kBlock / 32][kWarpCol];
+    const int lane = threadIdx.x & 31, c = term_comp();
+    unsigned char* ord = order[threadIdx.x >> 5];
+    // the tails in ascending id
+    column_order(n, lane < n ? __ldg(sprev + b + lane) : INT32_MAX, lane + 32 < n ? __ldg(sprev + b + lane + 32) : INT32_MAX,
+                 ord);
+    float nb[8], fp[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int k = 8 * j + term_slot();
+        nb[j] = fp[j] = 0.0f;
+        if (k < n) {
+            nb[j] = ldg1(P, __ldg(sprev + b + ord[k]), c);
+            fp[j] = ldg1(FP, fc.face(__ldg(sc + b + k)), c);
         }
-        float4 pn = f4_mul(ldg4(P, v), __fadd_rn((float)n, -2.0f));
-        y = f4_div_z(f4_add(f4_div_z(acc, (float)n), pn), (float)n);
-    } else {
-        float4 sh = f4_zero(), sl = f4_zero();
-        for (int k = 0; k < n; ++k) dd_acc(sh, sl, col4(f0, f1, k));
-        for (int r = 0; r < n; ++r) {
-            int src, el;
-            slot_of_rank(r, h0, h1, r0, r1, src, el);
-            dd_acc(sh, sl, shfl4(el ? p1 : p0, src));
-        }
-        y = vp_finish(sh, sl, ldg4(P, v), n);
     }
+    __syncwarp();
+    float4 y = column_point<true>(nb, fp, ldg1(P, v, c), n, compensated != 0);
     if (lane == 0) {
         if (boundary) y = vp_lak_boundary(sc, snext, sprev, sprevc, sflag, eid, P, v, b, b + n, y);
         st4(R, v, y);

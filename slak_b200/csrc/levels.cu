@@ -79,6 +79,7 @@ void launch_fast_t(const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc&
     FastDims d{(int)Pl.N, (int)Pl.V, (int)Pl.F, (int)Pl.E, (int)L.V, (int)L.N, (int)Pl.B};
     if (GQ || SG) { d.N2 = (int)L.gN; d.V2 = (int)L.gV; d.F2 = (int)L.gF; }
     const int nv3 = GQ ? (int)L.gV : (int)Pl.V;      // k_g3's vertices
+    const int mode = (comp ? G3_COMP : 0) | (L.longcol ? G3_LONG : 0);
     cudaStream_t str = lc.s;
     // compulsory bytes of each kernel: the level's corner ids and positions it
     // must read once, and the refined ids / positions it alone writes
@@ -122,7 +123,7 @@ void launch_fast_t(const Level& Pl, const Level& L, Faces<PQ> pf, bool comp, Lc&
     } else {
         with_block(L.bs[2], [&](auto b) {
             constexpr int BS = decltype(b)::value;
-            launch_g<k_g3_g<LAK, STATE, BS, BND, SG>>(grid_for(nv3 + 1, BS), BS, str, d, L.verts, L.in_state, L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv3, nullptr, 0);
+            launch_g<k_g3_g<LAK, STATE, BS, BND, SG>>(grid_for(nv3 + 1, BS), BS, str, d, L.verts, L.in_state, L.out_state, L.slots, L.o_verts, mode, nv3, nullptr, 0);
         });
     }
     // compulsory bytes: the vertex points of its vertices, SLAK the edge points of their slots
@@ -186,10 +187,11 @@ void launch_pp_t(const Level& PPl, const Level& Pl, const Level& L, Faces<PQ> pf
     lc.after("k_pp", 1, 16 * PPl.N + 16 * L.V + (wids ? 16 * L.N : 0) + 16 * L.Vo - g3 +
                             (optr ? 4 * (L.N + 1) + 16 * L.N : 0));
     const int nv = (int)(PQ ? PPl.V : PPl.V + PPl.F);
+    const int mode = (comp ? G3_COMP : 0) | (L.longcol ? G3_LONG : 0);
     with_block(L.bs[2], [&](auto b) {
         constexpr int BS = decltype(b)::value;
         launch_g<k_g3_g<LAK, STATE, BS, false, false, true>>(grid_for(nv + 1, BS), BS, lc.s, d, L.verts, L.in_state,
-                                                             L.out_state, L.slots, L.o_verts, comp ? 1 : 0, nv,
+                                                             L.out_state, L.slots, L.o_verts, mode, nv,
                                                              PQ ? nullptr : PPl.ptr, kPpFace);
     });
     lc.after("k_g3", 1, g3);

@@ -31,6 +31,7 @@ struct Level {
     // closed level with a grandparent (grand.cuh): refined from the
     // grandparent's state and the parent's quads
     bool pp = false;
+    bool longcol = false;        // the input has vertices above valence 15 (long columns at every level)
     bool skip_ids = false;       // its refined quads are read by no later level
     // k_g3 with bulk-copied slot records (SLAK_PLAN_BULK_RECORDS, closed parents)
     bool bulk3 = false;

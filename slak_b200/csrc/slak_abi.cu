@@ -618,6 +618,7 @@ int plan_levels(slak_plan* p)
             L.F = P.Fo; L.V = P.Vo; L.N = P.No; L.B = 2 * P.B;
             L.E = (L.N - L.B) / 2 + L.B;
             L.quad = true; L.poly_fn = false;
+            L.longcol = p->vhist[16] > 0;
             L.fast = !force_general;     // any parent: closed or open, quad or polygon faces
         }
         L.Fo = L.N; L.No = 4 * L.N; L.Vo = L.V + L.F + L.E;
