@@ -84,8 +84,9 @@ const char* slak_last_error_detail(void);
  * complete (the reference is synchronous too).  Intermediate levels live in a
  * per-device workspace that is kept for the next call (the reference
  * allocates and frees them inside every call); a call made while another
- * holds the workspace allocates its own.  SLAK_WORKSPACE_CACHE=0 in the
- * environment turns the cache off.
+ * holds the workspace allocates its own.  Output arrays that came back through
+ * slak_mesh_free are kept too, at most 1 GiB per device, and handed out again.
+ * SLAK_WORKSPACE_CACHE=0 in the environment turns both off.
  */
 int slak_subdivide(const slak_mesh* cmesh, slak_mesh* rmesh, int target_level, int scheme,
                    slak_stream_t stream);
@@ -147,13 +148,16 @@ int slak_obj_write_sharp(const char* path, const slak_mesh* host_mesh, const sla
                          const slak_corners* corners);
 int slak_obj_free_corners(slak_corners* corners);
 
-/* Frees the current device's cached slak_subdivide workspace.  No counterpart
- * in the reference, whose calls keep nothing between them.  Returns
- * SLAK_ERR_NOT_READY while a call holds the workspace. */
+/* Frees the current device's cached slak_subdivide workspace and the idle
+ * output arrays slak_mesh_free kept.  No counterpart in the reference, whose
+ * calls keep nothing between them.  Returns SLAK_ERR_NOT_READY while a call
+ * holds the workspace. */
 int slak_workspace_release(void);
 
 /* cudaFree of every non-NULL array, then zero the descriptor
- * (MeshInfo::freeAndReset, CatmullClark.h:99-106). */
+ * (MeshInfo::freeAndReset, CatmullClark.h:99-106).  Like cudaFree it waits for
+ * the device; arrays of slak_subdivide and slak_subdivide_batched may be kept
+ * idle for their next calls instead (see slak_subdivide). */
 int slak_mesh_free(slak_mesh* mesh);
 
 /*

@@ -63,6 +63,137 @@ struct Carver {
     }
 };
 
+// ------------------------------------------------------------------ results' memory
+// The one-shot calls hand their outputs to the caller (slak_mesh_free or
+// cudaFree).  cudaMalloc and cudaFree of one array cost 330 + 260 us on a B200
+// host (at any size up to 64 MiB), five to ten times the refinement of a small
+// mesh, so the arrays that slak_mesh_free gets back are kept, idle, for later
+// calls on the same device: at most kOutCacheBytes per device, returned by
+// slak_workspace_release and before an allocation of this library fails;
+// SLAK_WORKSPACE_CACHE=0 turns it off.  Only arrays these calls allocated are
+// kept; one the caller freed with cudaFree just leaves the table (its entry is
+// checked against the driver's allocation before it is believed).
+constexpr size_t kOutCacheBytes = size_t(1) << 30;
+constexpr int kWsMaxDevices = 64;
+
+struct OutBlock {
+    size_t bytes;
+    int dev;
+};
+std::mutex g_out_mu;
+std::map<void*, OutBlock> g_out_live;                                   // handed out
+std::multimap<size_t, void*> g_out_idle[kWsMaxDevices];                 // by size
+size_t g_out_idle_bytes[kWsMaxDevices] = {};
+
+bool workspace_cached()
+{
+    const char* env = std::getenv("SLAK_WORKSPACE_CACHE");
+    return !(env && env[0] == '0');
+}
+
+int current_device()
+{
+    int dev = -1;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kWsMaxDevices ? dev : -1;
+}
+
+// frees the device's idle blocks; true if there were any
+bool out_trim(int dev)
+{
+    std::vector<void*> v;
+    {
+        std::lock_guard<std::mutex> lk(g_out_mu);
+        for (const auto& e : g_out_idle[dev]) v.push_back(e.second);
+        g_out_idle[dev].clear();
+        g_out_idle_bytes[dev] = 0;
+    }
+    for (void* p : v) cudaFree(p);
+    return !v.empty();
+}
+
+// cudaMalloc that gives the idle blocks back before it fails
+cudaError_t device_malloc(void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    const int dev = e == cudaErrorMemoryAllocation ? current_device() : -1;
+    if (dev >= 0 && out_trim(dev)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+// an output array: the smallest idle block that holds it and is not twice its size
+cudaError_t out_malloc(void** p, size_t bytes)
+{
+    const int dev = workspace_cached() ? current_device() : -1;
+    if (dev >= 0) {
+        std::lock_guard<std::mutex> lk(g_out_mu);
+        auto it = g_out_idle[dev].lower_bound(bytes);
+        if (it != g_out_idle[dev].end() && it->first / 2 <= std::max(bytes, size_t(1) << 16)) {
+            *p = it->second;
+            g_out_idle_bytes[dev] -= it->first;
+            g_out_live[*p] = OutBlock{it->first, dev};
+            g_out_idle[dev].erase(it);
+            return cudaSuccess;
+        }
+    }
+    const cudaError_t e = device_malloc(p, bytes);
+    if (e == cudaSuccess && dev >= 0) {
+        std::lock_guard<std::mutex> lk(g_out_mu);
+        g_out_live[*p] = OutBlock{bytes, dev};
+    }
+    return e;
+}
+
+template <class T>
+cudaError_t out_malloc(T** p, size_t bytes)
+{
+    void* q = nullptr;
+    const cudaError_t e = out_malloc(&q, bytes);
+    if (e == cudaSuccess) *p = static_cast<T*>(q);
+    return e;
+}
+
+// cudaFree of an array that may be in the table
+cudaError_t out_free(void* p)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_out_mu);
+        g_out_live.erase(p);
+    }
+    return cudaFree(p);
+}
+
+// Keeps `p` idle instead of freeing it; false if it is not one of these
+// blocks (or no longer: the caller freed it and the address was allocated
+// again) or does not fit.  The device is idle (the caller synchronised).
+bool out_keep(void* p, int dev)
+{
+    static const auto range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr)>(f);
+    }();
+    std::lock_guard<std::mutex> lk(g_out_mu);
+    auto it = g_out_live.find(p);
+    if (it == g_out_live.end()) return false;
+    const OutBlock b = it->second;
+    g_out_live.erase(it);
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (b.dev != dev || range == nullptr || range(&base, &size, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS ||
+        base != reinterpret_cast<CUdeviceptr>(p) || size < b.bytes)
+        return false;
+    if (g_out_idle_bytes[dev] + b.bytes > kOutCacheBytes) return false;
+    g_out_idle[dev].emplace(b.bytes, p);
+    g_out_idle_bytes[dev] += b.bytes;
+    return true;
+}
+
 int cuda_status(cudaError_t e)
 {
     if (e == cudaSuccess) return SLAK_OK;
@@ -517,10 +648,10 @@ void free_plan_memory(slak_plan* p)
     if (p->h_st && p->h_st_owned) cudaFreeHost(p->h_st);
     p->h_st = nullptr;
     if (p->out_owned) {
-        if (p->out.ids) cudaFree(p->out.ids);
-        if (p->out.verts) cudaFree(p->out.verts);
-        if (p->out.ptr) cudaFree(p->out.ptr);
-        if (p->out.vals) cudaFree(p->out.vals);
+        if (p->out.ids) out_free(p->out.ids);
+        if (p->out.verts) out_free(p->out.verts);
+        if (p->out.ptr) out_free(p->out.ptr);
+        if (p->out.vals) out_free(p->out.vals);
     }
     std::memset(&p->out, 0, sizeof(p->out));
 }
@@ -785,22 +916,25 @@ struct Workspace {
     void* mem = nullptr;
     size_t bytes = 0;
     DevStatus* h_st = nullptr;
+    cudaStream_t side[2] = {nullptr, nullptr};      // for a level's independent kernels (110 us each to make)
+    cudaEvent_t cev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool busy = false;
 };
-constexpr int kWsMaxDevices = 64;
 std::mutex g_ws_mu;
 Workspace g_ws[kWsMaxDevices];
 
 Workspace* workspace_acquire()
 {
-    const char* env = std::getenv("SLAK_WORKSPACE_CACHE");
-    if (env && env[0] == '0') return nullptr;
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kWsMaxDevices) return nullptr;
+    const int dev = workspace_cached() ? current_device() : -1;
+    if (dev < 0) return nullptr;
     std::lock_guard<std::mutex> lk(g_ws_mu);
     Workspace* w = &g_ws[dev];
     if (w->busy) return nullptr;
     if (!w->h_st && cudaMallocHost(&w->h_st, sizeof(DevStatus)) != cudaSuccess) { w->h_st = nullptr; return nullptr; }
+    for (auto& st : w->side)
+        if (!st && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) { st = nullptr; return nullptr; }
+    for (auto& ev : w->cev)
+        if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) { ev = nullptr; return nullptr; }
     w->busy = true;
     return w;
 }
@@ -819,7 +953,7 @@ cudaError_t workspace_reserve(Workspace* w, size_t bytes)
     if (w->mem) cudaFree(w->mem);
     w->mem = nullptr;
     w->bytes = 0;
-    cudaError_t e = cudaMalloc(&w->mem, bytes);
+    cudaError_t e = device_malloc(&w->mem, bytes);
     if (e == cudaSuccess) w->bytes = bytes;
     return e;
 }
@@ -1033,7 +1167,11 @@ static int plan_create_impl(const slak_mesh* cm, int target_level, int scheme, i
     }
     rc = probe_level0(p, p->lv[0], str, probe_mem);
     if (rc == SLAK_OK) rc = plan_levels(p);
-    if (rc == SLAK_OK) {              // side streams for the levels' independent kernels
+    if (rc == SLAK_OK && ws) {        // side streams for the levels' independent kernels
+        std::copy(ws->side, ws->side + 2, p->side);
+        std::copy(ws->cev, ws->cev + 4, p->cev);
+        p->side_owned = false;
+    } else if (rc == SLAK_OK) {
         for (int k = 0; k < 2 && ce == cudaSuccess; ++k) ce = cudaStreamCreateWithFlags(&p->side[k], cudaStreamNonBlocking);
         for (int k = 0; k < 4 && ce == cudaSuccess; ++k) ce = cudaEventCreateWithFlags(&p->cev[k], cudaEventDisableTiming);
         if (ce != cudaSuccess) rc = cuda_status(ce);
@@ -1049,18 +1187,22 @@ static int plan_create_impl(const slak_mesh* cm, int target_level, int scheme, i
         p->arena = ws->mem;
         p->arena_owned = false;
     } else {
-        ce = cudaMalloc(&p->arena, dry.off);
+        ce = device_malloc(&p->arena, dry.off);
     }
     if (ce != cudaSuccess) { free_plan_memory(p); delete p; return cuda_status(ce); }
     Carver cv((char*)p->arena);
     plan_carve(p, cv);
     // final outputs (caller-ownable, one allocation each)
     slak_mesh o = plan_output_shape(p);
-    ce = cudaMalloc(&o.ids, sizeof(int) * (size_t)o.nnz);
-    if (ce == cudaSuccess) ce = cudaMalloc(&o.verts, sizeof(float) * 4 * (size_t)o.nverts);
-    if (ce == cudaSuccess && scheme == SLAK_SCHEME_LAK) {
-        ce = cudaMalloc(&o.ptr, sizeof(int) * (size_t)(o.nfaces + 1));
-        if (ce == cudaSuccess) ce = cudaMalloc(&o.vals, sizeof(int) * (size_t)o.nnz);
+    // (a one-shot call's come from the idle ones)
+    const auto out = [&](auto** q, size_t bytes) {
+        if (ce == cudaSuccess) ce = ws ? out_malloc(q, bytes) : device_malloc(reinterpret_cast<void**>(q), bytes);
+    };
+    out(&o.ids, sizeof(int) * (size_t)o.nnz);
+    out(&o.verts, sizeof(float) * 4 * (size_t)o.nverts);
+    if (scheme == SLAK_SCHEME_LAK) {
+        out(&o.ptr, sizeof(int) * (size_t)(o.nfaces + 1));
+        out(&o.vals, sizeof(int) * (size_t)o.nnz);
     }
     p->out = o;
     if (ce == cudaSuccess && p->crease_levels > 0) {   // the plan keeps its own copy of the creases
@@ -1319,18 +1461,32 @@ int slak_workspace_release(void)
     if (w->busy) return SLAK_ERR_NOT_READY;
     if (w->mem) e = cudaFree(w->mem);
     if (w->h_st) cudaFreeHost(w->h_st);
+    for (auto st : w->side) if (st) cudaStreamDestroy(st);
+    for (auto ev : w->cev) if (ev) cudaEventDestroy(ev);
     *w = Workspace{};
+    out_trim(dev);
     return cuda_status(e);
 }
 
 int slak_mesh_free(slak_mesh* m)
 {
     if (!m) return SLAK_ERR_INVALID_ARG;
+    // arrays of the one-shot calls are kept idle for later calls; as with
+    // cudaFree, whatever still uses them is waited for first
     cudaError_t e = cudaSuccess, t;
-    if (m->ptr) { t = cudaFree(m->ptr); if (t != cudaSuccess) e = t; }
-    if (m->ids) { t = cudaFree(m->ids); if (t != cudaSuccess) e = t; }
-    if (m->vals) { t = cudaFree(m->vals); if (t != cudaSuccess) e = t; }
-    if (m->verts) { t = cudaFree(m->verts); if (t != cudaSuccess) e = t; }
+    const bool any = m->ptr || m->ids || m->vals || m->verts;
+    const int dev = any && workspace_cached() ? current_device() : -1;
+    if (dev >= 0) e = cudaDeviceSynchronize();
+    const bool keep = dev >= 0 && e == cudaSuccess;
+    const auto give = [&](void* p) {
+        if (!p || (keep && out_keep(p, dev))) return;
+        t = out_free(p);
+        if (t != cudaSuccess) e = t;
+    };
+    give(m->ptr);
+    give(m->ids);
+    give(m->vals);
+    give(m->verts);
     std::memset(m, 0, sizeof(*m));
     return cuda_status(e);
 }
@@ -1420,10 +1576,10 @@ void batch_free(slak_batch* b)
         for (size_t i = 0; i < b->outs.size(); ++i)
             if (!b->out_given[i]) {
                 slak_mesh& m = b->outs[i];
-                if (m.ids) cudaFree(m.ids);
-                if (m.verts) cudaFree(m.verts);
-                if (m.ptr) cudaFree(m.ptr);
-                if (m.vals) cudaFree(m.vals);
+                if (m.ids) out_free(m.ids);
+                if (m.verts) out_free(m.verts);
+                if (m.ptr) out_free(m.ptr);
+                if (m.vals) out_free(m.vals);
             }
     if (b->arena) cudaFree(b->arena);
     if (b->gmem) cudaFree(b->gmem);
@@ -1843,11 +1999,11 @@ static int batch_create_impl(const slak_mesh* meshes, const int* levels, int64_t
         for (int64_t i = 0; i < count && ce == cudaSuccess; ++i) {
             if (!b->plans[i]) continue;
             slak_mesh& m = b->outs[i];
-            ce = cudaMalloc(&m.ids, sizeof(int) * (size_t)m.nnz);
-            if (ce == cudaSuccess) ce = cudaMalloc(&m.verts, sizeof(float) * 4 * (size_t)m.nverts);
+            ce = out_malloc(&m.ids, sizeof(int) * (size_t)m.nnz);
+            if (ce == cudaSuccess) ce = out_malloc(&m.verts, sizeof(float) * 4 * (size_t)m.nverts);
             if (ce == cudaSuccess && scheme == SLAK_SCHEME_LAK) {
-                ce = cudaMalloc(&m.ptr, sizeof(int) * (size_t)(m.nfaces + 1));
-                if (ce == cudaSuccess) ce = cudaMalloc(&m.vals, sizeof(int) * (size_t)m.nnz);
+                ce = out_malloc(&m.ptr, sizeof(int) * (size_t)(m.nfaces + 1));
+                if (ce == cudaSuccess) ce = out_malloc(&m.vals, sizeof(int) * (size_t)m.nnz);
             }
         }
         if (ce != cudaSuccess) rc = cuda_status(ce);
