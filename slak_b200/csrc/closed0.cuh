@@ -69,7 +69,8 @@ template <bool QUAD, bool LAK, bool CAP>
 __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* __restrict__ ptr,
                                                 const int* __restrict__ ids, int F, int N, int V,
                                                 const float* __restrict__ P, float* __restrict__ FP,
-                                                int* __restrict__ cface, unsigned long long* __restrict__ cnt,
+                                                int* __restrict__ cface, unsigned* __restrict__ nav,
+                                                unsigned long long* __restrict__ cnt,
                                                 int* __restrict__ rank, int4* __restrict__ rec, DevStatus* st)
 {
     const int f = bx_ * kBlock + threadIdx.x;
@@ -106,6 +107,7 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
                 if (k < n) {
                     const int w = k + 1 < n ? v[(k + 1) & 7] : v[0], u = k ? v[(k + 7) & 7] : last;
                     cface[b + k] = f;
+                    nav[b + k] = (unsigned)k | ((unsigned)(n - 1 - k) << 16);
                     c0_corner<LAK, CAP>(b + k, f, v[k], w, u, k == 0, V, cnt, rank, rec, st);
                 }
 #pragma unroll
@@ -116,6 +118,7 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
             for (int c = b; c < e; ++c) {
                 const int w = __ldg(ids + (c + 1 < e ? c + 1 : b));
                 cface[c] = f;
+                nav[c] = n <= 0xffff ? (unsigned)(c - b) | ((unsigned)(e - 1 - c) << 16) : kNavFar;
                 c0_corner<LAK, CAP>(c, f, v, w, u, c == b, V, cnt, rank, rec, st);
                 acc = f4_add(acc, pos(v));
                 u = v;
@@ -128,11 +131,12 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
 template <bool QUAD, bool LAK, bool CAP>
 __global__ void __launch_bounds__(kBlock) k_c0_faces(const int* __restrict__ ptr, const int* __restrict__ ids, int F,
                                                      int N, int V, const float* __restrict__ P, float* __restrict__ FP,
-                                                     int* __restrict__ cface, unsigned long long* __restrict__ cnt,
+                                                     int* __restrict__ cface, unsigned* __restrict__ nav,
+                                                     unsigned long long* __restrict__ cnt,
                                                      int* __restrict__ rank, int4* __restrict__ rec, DevStatus* st)
 {
     griddep_enter();
-    k_c0_faces_body<QUAD, LAK, CAP>(blockIdx.x, ptr, ids, F, N, V, P, FP, cface, cnt, rank, rec, st);
+    k_c0_faces_body<QUAD, LAK, CAP>(blockIdx.x, ptr, ids, F, N, V, P, FP, cface, nav, cnt, rank, rec, st);
 }
 template <bool QUAD, bool LAK, bool CAP>
 struct k_c0_faces_g {
@@ -277,9 +281,7 @@ __device__ __forceinline__ void c0_nav(const Faces<QUAD>& fc, int c, int N, int 
     } else {
         f = __ldg(fc.cface + c);
         if ((unsigned)f >= (unsigned)F) f = 0;
-        const int b = __ldg(fc.ptr + f), e = __ldg(fc.ptr + f + 1);
-        nc = c + 1 < e ? c + 1 : b;
-        p = c > b ? c - 1 : e - 1;
+        fc.around(c, nc, p);
         if ((unsigned)nc >= (unsigned)N) nc = c;
         if ((unsigned)p >= (unsigned)N) p = c;
     }
@@ -327,7 +329,7 @@ struct k_c0_bucket_g {
 // What a vertex pass writes: corner -> slot / twin / edge id; the slot-ordered
 // column (sc, snext, sprev, sprevc) of long columns, and of all with creases.
 struct C0Out {
-    int *xslot, *xtw, *eid;
+    int *xslot, *xtw, *xnt, *eid;        // (xnt: next(twin))
     int *sc, *snext, *sprev, *sprevc, *sflag;
     int all;                // every column's slots are wanted (creases)
 };
@@ -338,33 +340,6 @@ __device__ __forceinline__ int rec_prev(const int* __restrict__ ptr, int4 r)
     if (QUAD) return (r.x & ~3) | ((r.x + 3) & 3);
     return r.y < 0 ? __ldg(ptr + r.w + 1) - 1 : r.x - 1;
 }
-__device__ __forceinline__ void rec_cswap(int4& a, int4& b)
-{
-    const bool s = b.x < a.x;
-    const int4 t = a;
-    a.x = s ? b.x : a.x; a.y = s ? b.y : a.y; a.z = s ? b.z : a.z; a.w = s ? b.w : a.w;
-    b.x = s ? t.x : b.x; b.y = s ? t.y : b.y; b.z = s ? t.z : b.z; b.w = s ? t.w : b.w;
-}
-
-__device__ __forceinline__ void rec_cswap(int& a, int& b)
-{
-    const int lo = min(a, b);
-    b = max(a, b);
-    a = lo;
-}
-// sorting networks of 4 and 8 (Batcher's odd-even merge)
-template <int NMAX, class T>
-__device__ __forceinline__ void sort_keys(T (&r)[NMAX])
-{
-    rec_cswap(r[0], r[1]); rec_cswap(r[2], r[3]); rec_cswap(r[0], r[2]); rec_cswap(r[1], r[3]); rec_cswap(r[1], r[2]);
-    if constexpr (NMAX == 8) {
-        rec_cswap(r[4], r[5]); rec_cswap(r[6], r[7]); rec_cswap(r[4], r[6]); rec_cswap(r[5], r[7]); rec_cswap(r[5], r[6]);
-        rec_cswap(r[0], r[4]); rec_cswap(r[1], r[5]); rec_cswap(r[2], r[6]); rec_cswap(r[3], r[7]);
-        rec_cswap(r[2], r[4]); rec_cswap(r[3], r[5]);
-        rec_cswap(r[1], r[2]); rec_cswap(r[3], r[4]); rec_cswap(r[5], r[6]);
-    }
-}
-
 // One vertex of n <= NMAX corners (records rec, unsorted) on its own thread.
 template <bool QUAD, bool LAK, int NMAX>
 __device__ __forceinline__ void c0_vertex(const int* __restrict__ ptr, const int4* __restrict__ rec, int v, int b,
@@ -397,11 +372,11 @@ __device__ __forceinline__ void c0_vertex(const int* __restrict__ ptr, const int
     for (int k = 0; k < NMAX; ++k) {
         if (k >= n) continue;
         const int w = nx[k], c = r[k].x;
-        int tw = -1, less = 0;
+        int tw = -1, nt = c, less = 0;
 #pragma unroll
         for (int t = 0; t < NMAX; ++t) {
             if (t >= n) continue;
-            if (r[t].z == w) { if (tw < 0) tw = pc[t]; else bad = 1; }
+            if (r[t].z == w) { if (tw < 0) { tw = pc[t]; nt = r[t].x; } else bad = 1; }
             if (t < k && nx[t] == w) bad = 1;
             less += nx[t] < w;
         }
@@ -409,6 +384,7 @@ __device__ __forceinline__ void c0_vertex(const int* __restrict__ ptr, const int
         const int twc = tw < 0 ? c : tw;
         o.xslot[c] = b + k;
         o.xtw[c] = twc;
+        if (!QUAD) o.xnt[c] = nt;
         if (LAK ? w < v : v < w) {
             int id = id0 + (LAK ? less : own);
             if ((unsigned)id >= (unsigned)E) { bad = 1; id = 0; }
@@ -505,6 +481,7 @@ __device__ __forceinline__ void k_c0_verts_body(const unsigned bx_, const int* _
                 const int s = bb + rk;
                 o.xslot[me.x] = s;
                 o.xtw[me.x] = tw < 0 ? me.x : tw;
+                if (!QUAD) o.xnt[me.x] = hit.x < 0 ? me.x : hit.x;
                 o.sc[s] = me.x;
                 o.snext[s] = w;
                 o.sprev[s] = me.z;

@@ -417,6 +417,34 @@ __device__ __forceinline__ void rank_order(const int* __restrict__ key, int b, i
     }
 }
 
+// ---------------------------------------------------------------- small sorts
+__device__ __forceinline__ void key_cswap(int4& a, int4& b)
+{
+    const bool s = b.x < a.x;
+    const int4 t = a;
+    a.x = s ? b.x : a.x; a.y = s ? b.y : a.y; a.z = s ? b.z : a.z; a.w = s ? b.w : a.w;
+    b.x = s ? t.x : b.x; b.y = s ? t.y : b.y; b.z = s ? t.z : b.z; b.w = s ? t.w : b.w;
+}
+
+__device__ __forceinline__ void key_cswap(int& a, int& b)
+{
+    const int lo = min(a, b);
+    b = max(a, b);
+    a = lo;
+}
+// sorting networks of 4 and 8 (Batcher's odd-even merge)
+template <int NMAX, class T>
+__device__ __forceinline__ void sort_keys(T (&r)[NMAX])
+{
+    key_cswap(r[0], r[1]); key_cswap(r[2], r[3]); key_cswap(r[0], r[2]); key_cswap(r[1], r[3]); key_cswap(r[1], r[2]);
+    if constexpr (NMAX == 8) {
+        key_cswap(r[4], r[5]); key_cswap(r[6], r[7]); key_cswap(r[4], r[6]); key_cswap(r[5], r[7]); key_cswap(r[5], r[6]);
+        key_cswap(r[0], r[4]); key_cswap(r[1], r[5]); key_cswap(r[2], r[6]); key_cswap(r[3], r[7]);
+        key_cswap(r[2], r[4]); key_cswap(r[3], r[5]);
+        key_cswap(r[1], r[2]); key_cswap(r[3], r[4]); key_cswap(r[5], r[6]);
+    }
+}
+
 // ---------------------------------------------------------------- status
 // Device-side status written by kernels; the host reads it after a sync.
 struct DevStatus {
@@ -437,11 +465,26 @@ __device__ __forceinline__ void set_error(DevStatus* st, int code, int detail)
 // Corner navigation: QUAD uses the implicit 4-corner faces of the reference's
 // quad functions (`threadId / 4 * 4 + (threadId + 1) % 4`,
 // CatmullClarkKernels.cuh:155); otherwise face offsets + a corner->face map.
+constexpr unsigned kNavFar = 0xffffffffu;
 template <bool QUAD>
 struct Faces {
     const int* __restrict__ ptr;
     const int* __restrict__ cface;
+    const unsigned* __restrict__ nav = nullptr;     // corners before c in its face | after it << 16 (kNavFar: use ptr)
     __device__ __forceinline__ int face(int c) const { return QUAD ? (c >> 2) : __ldg(cface + c); }
+    // next and previous corner, with `nav`: one load instead of the face's two offsets behind its id
+    __device__ __forceinline__ void around(int c, int& nc, int& pc) const
+    {
+        const unsigned u = QUAD || nav == nullptr ? kNavFar : __ldg(nav + c);
+        if (u != kNavFar) {
+            const int before = (int)(u & 0xffffu), after = (int)(u >> 16);
+            nc = after ? c + 1 : c - before;
+            pc = before ? c - 1 : c + after;
+        } else {
+            nc = next(c);
+            pc = prev(c);
+        }
+    }
     __device__ __forceinline__ int next(int c) const
     {
         if (QUAD) return (c & ~3) | ((c + 1) & 3);

@@ -62,6 +62,7 @@ struct QState {
     int* tw;       // -1: no twin (boundary half-edge)
     int* t;        // -1: the previous corner's half-edge has no twin
     int* brank;    // per edge: boundary edges with a smaller id (meshes with a boundary)
+    int* nt;       // next(tw) (closed polygon input)
 };
 
 struct FastDims {

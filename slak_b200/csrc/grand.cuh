@@ -188,15 +188,16 @@ __device__ __forceinline__ void k_pp_body(const unsigned bx_, FastDims d, Faces<
         vn = __shfl_sync(full, q.x, ln);
         if (LAK) vp = __shfl_sync(full, q.x, lp);
     } else {
-        const int face = q.z - d.V2;
-        fb = __ldg(pf.ptr + face); fe = __ldg(pf.ptr + face + 1);
+        const unsigned u = __ldg(pf.nav + y);
+        if (u != kNavFar) { fb = y - (int)(u & 0xffffu); fe = y + 1 + (int)(u >> 16); }
+        else { fb = __ldg(pf.ptr + q.z - d.V2); fe = __ldg(pf.ptr + q.z - d.V2 + 1); }
         ny = y + 1 == fe ? fb : y + 1;
         py = y == fb ? fe - 1 : y - 1;
         twp = __ldg(pp.tw + py);
         vn = __ldg(&pids[ny].x);
         qp = __ldg(pids + py);
         vp = qp.x;
-        nh2 = pf.next(tw);
+        nh2 = __ldg(pp.nt + y);
     }
     const int ee = q.y - VF2, ep = q.w - VF2;              // PP's edges through y and prev(y)
     // P's edges of the P face: v-eo, eo-f, f-ei, ei-v
@@ -215,7 +216,11 @@ __device__ __forceinline__ void k_pp_body(const unsigned bx_, FastDims d, Faces<
     } else {
         int vnn;
         if constexpr (PQ) vnn = __ldg(&pids[qnext(nh2)].x);
-        else vnn = __ldg(&pids[pf.next(nh2)].x);
+        else {
+            int nn2, pn2;
+            pf.around(nh2, nn2, pn2);
+            vnn = __ldg(&pids[nn2].x);
+        }
         EW = 4 * (__ldg(&pids[nh2].y) - VF2) + (q.x > vnn);
     }
     const bool own = valid && q.x < vn;                     // sums PP's edge point eo's column

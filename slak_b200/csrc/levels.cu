@@ -8,6 +8,7 @@
 
 #include "plan.cuh"
 #include "grand.cuh"
+#include "poly1.cuh"
 
 namespace slak {
 namespace {
@@ -227,9 +228,56 @@ void launch_fast_gq(const Level& Pl, const Level& L, bool lak, bool comp, Lc& lc
     launch_fast_p<true, false, true>(Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
 }
 #elif SLAK_UNIT == 4
-void launch_fast_poly(const Level& Pl, const Level& L, const int* cface, bool lak, bool comp, Lc& lc)
+// Level 1 of a closed polygon input (poly1.cuh): C = L, its parent Pl the
+// input.  k_p1 runs blocks of bs[0] / 2 threads; bs[1] picks its register cap
+// (128, 256, 512: for 1024, 768, 512 resident threads).
+template <bool LAK, bool STATE>
+static void launch_p1_t(const Level& Pl, const Level& L, Faces<false> pf, bool comp, Lc& lc)
 {
-    launch_fast_p<false, false>(Pl, L, Faces<false>{Pl.ptr, cface}, lak, comp, lc);
+    FastDims d{(int)Pl.N, (int)Pl.V, (int)Pl.F, (int)Pl.E, (int)L.V, (int)L.N, 0};
+    int* optr = LAK && !STATE ? L.o_ptr : nullptr;
+    int4* ovals = LAK && !STATE ? reinterpret_cast<int4*>(L.o_vals) : nullptr;
+    const int mode = (comp ? G3_COMP : 0) | (L.longcol ? G3_LONG : 0);
+    bool mapped = true;
+    with_block(L.bs[0], [&](auto b) {
+        constexpr int BS = decltype(b)::value / 2;
+        CUtensorMap otm;
+        std::memset(&otm, 0, sizeof otm);
+        if (!STATE) mapped = quad_store_map(otm, L.o_ids, Pl.N, BS);
+        if (!mapped) return;            // nothing of the level is launched
+        with_block(L.bs[1], [&](auto r) {
+            constexpr int RT = decltype(r)::value == 128 ? 1024 : decltype(r)::value == 256 ? 768 : 512;
+            const unsigned nb = grid_for(L.F, BS);
+            launch_g<k_p1_g<LAK, STATE, BS, RT>>(nb + grid_for(Pl.F, BS), BS, lc.s, d, pf,
+                                                 reinterpret_cast<const int4*>(L.ids), L.verts, L.in_state, L.out_state,
+                                                 reinterpret_cast<int4*>(L.o_ids), otm, L.o_verts, L.slots, optr,
+                                                 ovals, comp ? 1 : 0, (int)nb);
+        });
+    });
+    if (!mapped) {
+        if (!lc.err) lc.err = SLAK_ERR_CUDA;
+        return;
+    }
+    const int64_t g3 = 16 * Pl.V + (LAK ? 0 : 16 * L.F);
+    lc.after("k_p1", 1, 4 * L.N + 16 * L.V + (L.skip_ids ? 0 : 16 * L.N) + 16 * L.Vo - g3 +
+                            (optr ? 4 * (L.N + 1) + 16 * L.N : 0));
+    with_block(L.bs[2], [&](auto b) {
+        constexpr int BS = decltype(b)::value;
+        launch_g<k_g3_g<LAK, STATE, BS>>(grid_for(Pl.V + 1, BS), BS, lc.s, d, L.verts, L.in_state, L.out_state, L.slots,
+                                         L.o_verts, mode, (int)Pl.V, nullptr, 0);
+    });
+    lc.after("k_g3", 1, g3);
+}
+
+void launch_p1(const Level& Pl, const Level& L, Faces<false> pf, bool lak, bool comp, Lc& lc)
+{
+    if (lak) {
+        if (L.make_state) launch_p1_t<true, true>(Pl, L, pf, comp, lc);
+        else launch_p1_t<true, false>(Pl, L, pf, comp, lc);
+    } else {
+        if (L.make_state) launch_p1_t<false, true>(Pl, L, pf, comp, lc);
+        else launch_p1_t<false, false>(Pl, L, pf, comp, lc);
+    }
 }
 #elif SLAK_UNIT == 5
 void launch_fast_poly_open(const Level& Pl, const Level& L, const int* cface, bool lak, bool comp, Lc& lc)
@@ -242,9 +290,9 @@ void launch_pp_quad(const Level& PPl, const Level& Pl, const Level& L, bool lak,
     launch_pp<true>(PPl, Pl, L, Faces<true>{nullptr, nullptr}, lak, comp, lc);
 }
 #elif SLAK_UNIT == 7
-void launch_pp_poly(const Level& PPl, const Level& Pl, const Level& L, const int* cface, bool lak, bool comp, Lc& lc)
+void launch_pp_poly(const Level& PPl, const Level& Pl, const Level& L, Faces<false> pf, bool lak, bool comp, Lc& lc)
 {
-    launch_pp<false>(PPl, Pl, L, Faces<false>{PPl.ptr, cface}, lak, comp, lc);
+    launch_pp<false>(PPl, Pl, L, pf, lak, comp, lc);
 }
 #endif
 

@@ -118,15 +118,15 @@ struct Lc {
     }
 };
 
-// the closed-form levels by parent kind (levels.cu; `cface`: the polygon
-// parent's or grandparent's corner -> face map)
+// the closed-form levels by parent kind (levels.cu; `cface` / `pf`: the polygon
+// parent's or grandparent's corner -> face map / faces)
 void launch_fast_quad(const Level& Pl, const Level& L, bool lak, bool comp, Lc& lc);
 void launch_fast_quad_open(const Level& Pl, const Level& L, bool lak, bool comp, Lc& lc);
 void launch_fast_gq(const Level& Pl, const Level& L, bool lak, bool comp, Lc& lc);
-void launch_fast_poly(const Level& Pl, const Level& L, const int* cface, bool lak, bool comp, Lc& lc);
+void launch_p1(const Level& Pl, const Level& L, Faces<false> pf, bool lak, bool comp, Lc& lc);
 void launch_fast_poly_open(const Level& Pl, const Level& L, const int* cface, bool lak, bool comp, Lc& lc);
 void launch_pp_quad(const Level& PPl, const Level& Pl, const Level& L, bool lak, bool comp, Lc& lc);
-void launch_pp_poly(const Level& PPl, const Level& Pl, const Level& L, const int* cface, bool lak, bool comp, Lc& lc);
+void launch_pp_poly(const Level& PPl, const Level& Pl, const Level& L, Faces<false> pf, bool lak, bool comp, Lc& lc);
 
 // exclusive scan of n counts (n + 1 outputs; scan.cuh), returns its launches
 int scan_launch(const int* in, int* out, int64_t n, int* tmp, cudaStream_t s);

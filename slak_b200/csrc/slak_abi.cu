@@ -42,8 +42,9 @@ struct Scratch {
     // closed level 0 (closed0.cuh): both counts per vertex, their tile sums, the
     // corners' ranks and records
     u64 *cnt2 = nullptr, *tmp2 = nullptr;
-    int* rank = nullptr;
+    int *rank = nullptr, *xnt = nullptr;
     int4* rec = nullptr;
+    unsigned* nav = nullptr;
 };
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -288,6 +289,8 @@ void carve_closed0(Carver& cv, Scratch& s, int64_t N, int64_t V, bool poly, bool
     s.cnt2 = cv.take<u64>(V);
     s.tmp2 = cv.take<u64>(scan_tiles(V) + 1);
     s.cface = poly ? cv.take<int>(N) : nullptr;
+    s.nav = poly ? cv.take<unsigned>(N) : nullptr;
+    s.xnt = poly ? cv.take<int>(N) : nullptr;
     s.sptr = cv.take<int>(V + 1);
     s.eptr = cv.take<int>(V + 1);
     s.rank = cap ? nullptr : cv.take<int>(N);
@@ -440,23 +443,23 @@ void launch_rest(const Level& L, int li, int scheme, bool compensated, Scratch& 
     if (lc.conc) { lc.join(0); lc.join(1); }
 }
 
-// `L` is the level, L[-1] its parent; `cface` is level 0's corner -> face map
-// when it has polygon faces
-void launch_fast(const Level* Lp, const int* cface, int scheme, bool comp, Lc& lc)
+// `L` is the level, L[-1] its parent; `cface` / `nav` are level 0's corner -> face
+// map and corner positions (Faces) when it has polygon faces
+void launch_fast(const Level* Lp, const int* cface, const unsigned* nav, int scheme, bool comp, Lc& lc)
 {
     const Level &L = *Lp, &Pl = Lp[-1];
     const bool lak = scheme == SLAK_SCHEME_LAK;
     if (L.pp) {
         const Level& PPl = Lp[-2];
         if (PPl.quad) launch_pp_quad(PPl, Pl, L, lak, comp, lc);
-        else launch_pp_poly(PPl, Pl, L, cface, lak, comp, lc);
+        else launch_pp_poly(PPl, Pl, L, Faces<false>{PPl.ptr, cface, nav}, lak, comp, lc);
         return;
     }
     if (L.gq) launch_fast_gq(Pl, L, lak, comp, lc);
     else if (Pl.quad && Pl.B > 0) launch_fast_quad_open(Pl, L, lak, comp, lc);
     else if (Pl.quad) launch_fast_quad(Pl, L, lak, comp, lc);
     else if (Pl.B > 0) launch_fast_poly_open(Pl, L, cface, lak, comp, lc);
-    else launch_fast_poly(Pl, L, cface, lak, comp, lc);
+    else launch_p1(Pl, L, Faces<false>{Pl.ptr, cface, nav}, lak, comp, lc);
 }
 
 // A closed level 0 (closed0.cuh); its counts s.cnt2 are zero.
@@ -465,11 +468,11 @@ void launch_closed0_t(const Level& L, bool creased, bool comp, Scratch& s, DevSt
 {
     const int F = (int)L.F, V = (int)L.V, N = (int)L.N, E = (int)L.E;
     cudaStream_t str = lc.s;
-    Faces<QUAD> fc{L.ptr, s.cface};
+    Faces<QUAD> fc{L.ptr, s.cface, s.nav};
     float* R = L.o_verts;
     float* FPo = R + 4 * (size_t)V;
     float* EPo = R + 4 * ((size_t)V + (size_t)F);
-    launch_g<k_c0_faces_g<QUAD, LAK, CAP>>(grid_for(F), kBlock, str, L.ptr, L.ids, F, N, V, L.verts, FPo, s.cface, s.cnt2,
+    launch_g<k_c0_faces_g<QUAD, LAK, CAP>>(grid_for(F), kBlock, str, L.ptr, L.ids, F, N, V, L.verts, FPo, s.cface, s.nav, s.cnt2,
                                            s.rank, s.rec, st);
     lc.after("k_c0_faces");
     const int nt = (int)std::max<int64_t>(1, scan_tiles(V));
@@ -486,7 +489,7 @@ void launch_closed0_t(const Level& L, bool creased, bool comp, Scratch& s, DevSt
         launch_g<k_c0_bucket_g<QUAD>>(grid_for(N), kBlock, str, fc, L.ids, N, F, V, s.sptr, s.rank, s.rec);
         lc.after("k_c0_bucket");
     }
-    const C0Out o{s.xslot, s.xtw, s.eid, s.sc, s.snext, s.sprev, s.sprevc, s.sflag, creased ? 1 : 0};
+    const C0Out o{s.xslot, s.xtw, s.xnt, s.eid, s.sc, s.snext, s.sprev, s.sprevc, s.sflag, creased ? 1 : 0};
     launch_g<k_c0_verts_g<QUAD, LAK, CAP>>(grid_for(V, 128), 128, str, L.ptr, V, E, s.sptr, s.eptr, s.rec, o, L.verts,
                                            FPo, R, comp ? 1 : 0, st);
     lc.after("k_c0_verts");
@@ -597,7 +600,7 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
         const Level& L = p->lv[li];
         lc.level = (int)li;
         if (L.fast) {
-            launch_fast(&L, p->s.cface, p->scheme, comp, lc);
+            launch_fast(&L, p->s.cface, p->s.nav, p->scheme, comp, lc);
             if (lc.err) break;          // a level that could not be launched stops the plan
             if ((int)li < p->crease_levels) launch_creases(p, (int)li, lc);
             continue;
@@ -896,7 +899,7 @@ void plan_wire(slak_plan* p)
         const Level& P = p->lv[i - 1];
         // the parent's state, or (SG, PP) the grandparent's
         const Level& S = p->lv[L.sg || L.pp ? i - 2 : i - 1];
-        if (S.export_state) L.in_state = QState{p->s.sptr, p->s.xslot, p->s.xtw, p->s.xt, p->s.xbrank};
+        if (S.export_state) L.in_state = QState{p->s.sptr, p->s.xslot, p->s.xtw, p->s.xt, p->s.xbrank, p->s.xnt};
         else L.in_state = S.out_state;
         if (L.make_state) L.out_state = p->qs[i];
         L.slots = p->slots;
@@ -1077,7 +1080,8 @@ int plan_autotune(slak_plan* p, cudaStream_t str)
                 for (int r = 0; r < 3 && rc == SLAK_OK; ++r) {
                     rc = enqueue_all(p, str);
                     if (rc == SLAK_OK) rc = cuda_status(cudaStreamSynchronize(str));
-                    t[r] = kernel_ms(p, li, k == 0 && L.pp ? "k_pp" : kTuneKernels[k]);
+                    const bool p1 = li == 1 && !p->lv[0].quad && p->lv[0].closed0;      // k_p1 (poly1.cuh)
+                    t[r] = kernel_ms(p, li, k < 2 && p1 ? "k_p1" : k == 0 && L.pp ? "k_pp" : kTuneKernels[k]);
                 }
                 std::sort(t, t + 3);
                 L.tune_ms[k][ci] = t[1];
