@@ -432,6 +432,12 @@ __device__ __forceinline__ void key_cswap(int& a, int& b)
     b = max(a, b);
     a = lo;
 }
+__device__ __forceinline__ void key_cswap(unsigned long long& a, unsigned long long& b)
+{
+    const unsigned long long lo = min(a, b);
+    b = max(a, b);
+    a = lo;
+}
 // sorting networks of 4 and 8 (Batcher's odd-even merge)
 template <int NMAX, class T>
 __device__ __forceinline__ void sort_keys(T (&r)[NMAX])
