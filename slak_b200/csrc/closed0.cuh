@@ -107,7 +107,7 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
                 if (k < n) {
                     const int w = k + 1 < n ? v[(k + 1) & 7] : v[0], u = k ? v[(k + 7) & 7] : last;
                     cface[b + k] = f;
-                    nav[b + k] = (unsigned)k | ((unsigned)(n - 1 - k) << 16);
+                    if (nav != nullptr) nav[b + k] = (unsigned)k | ((unsigned)(n - 1 - k) << 16);
                     c0_corner<LAK, CAP>(b + k, f, v[k], w, u, k == 0, V, cnt, rank, rec, st);
                 }
 #pragma unroll
@@ -118,7 +118,7 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
             for (int c = b; c < e; ++c) {
                 const int w = __ldg(ids + (c + 1 < e ? c + 1 : b));
                 cface[c] = f;
-                nav[c] = n <= 0xffff ? (unsigned)(c - b) | ((unsigned)(e - 1 - c) << 16) : kNavFar;
+                if (nav != nullptr) nav[c] = n <= 0xffff ? (unsigned)(c - b) | ((unsigned)(e - 1 - c) << 16) : kNavFar;
                 c0_corner<LAK, CAP>(c, f, v, w, u, c == b, V, cnt, rank, rec, st);
                 acc = f4_add(acc, pos(v));
                 u = v;
@@ -329,7 +329,7 @@ struct k_c0_bucket_g {
 // What a vertex pass writes: corner -> slot / twin / edge id; the slot-ordered
 // column (sc, snext, sprev, sprevc) of long columns, and of all with creases.
 struct C0Out {
-    int *xslot, *xtw, *xnt, *eid;        // (xnt: next(twin))
+    int *xslot, *xtw, *xnt, *eid;        // (xnt: next(twin), where another level follows a polygon mesh)
     int *sc, *snext, *sprev, *sprevc, *sflag;
     int all;                // every column's slots are wanted (creases)
 };
@@ -384,7 +384,7 @@ __device__ __forceinline__ void c0_vertex(const int* __restrict__ ptr, const int
         const int twc = tw < 0 ? c : tw;
         o.xslot[c] = b + k;
         o.xtw[c] = twc;
-        if (!QUAD) o.xnt[c] = nt;
+        if (!QUAD && o.xnt != nullptr) o.xnt[c] = nt;
         if (LAK ? w < v : v < w) {
             int id = id0 + (LAK ? less : own);
             if ((unsigned)id >= (unsigned)E) { bad = 1; id = 0; }
@@ -481,7 +481,7 @@ __device__ __forceinline__ void k_c0_verts_body(const unsigned bx_, const int* _
                 const int s = bb + rk;
                 o.xslot[me.x] = s;
                 o.xtw[me.x] = tw < 0 ? me.x : tw;
-                if (!QUAD) o.xnt[me.x] = hit.x < 0 ? me.x : hit.x;
+                if (!QUAD && o.xnt != nullptr) o.xnt[me.x] = hit.x < 0 ? me.x : hit.x;
                 o.sc[s] = me.x;
                 o.snext[s] = w;
                 o.sprev[s] = me.z;

@@ -284,13 +284,13 @@ void carve_scratch(Carver& cv, Scratch& s, int64_t N, int64_t V, int64_t E, bool
 
 // scratch of a closed level 0: `cap` no vertex above valence kC0Cap, `slots`
 // the slot-ordered columns are wanted (long columns, creases)
-void carve_closed0(Carver& cv, Scratch& s, int64_t N, int64_t V, bool poly, bool cap, bool slots)
+void carve_closed0(Carver& cv, Scratch& s, int64_t N, int64_t V, bool poly, bool cap, bool slots, bool state)
 {
     s.cnt2 = cv.take<u64>(V);
     s.tmp2 = cv.take<u64>(scan_tiles(V) + 1);
     s.cface = poly ? cv.take<int>(N) : nullptr;
-    s.nav = poly ? cv.take<unsigned>(N) : nullptr;
-    s.xnt = poly ? cv.take<int>(N) : nullptr;
+    s.nav = poly && state ? cv.take<unsigned>(N) : nullptr;     // (one level: not worth writing)
+    s.xnt = poly && state ? cv.take<int>(N) : nullptr;
     s.sptr = cv.take<int>(V + 1);
     s.eptr = cv.take<int>(V + 1);
     s.rank = cap ? nullptr : cv.take<int>(N);
@@ -468,11 +468,11 @@ void launch_closed0_t(const Level& L, bool creased, bool comp, Scratch& s, DevSt
 {
     const int F = (int)L.F, V = (int)L.V, N = (int)L.N, E = (int)L.E;
     cudaStream_t str = lc.s;
-    Faces<QUAD> fc{L.ptr, s.cface, s.nav};
+    Faces<QUAD> fc{L.ptr, s.cface, L.export_state ? s.nav : nullptr};
     float* R = L.o_verts;
     float* FPo = R + 4 * (size_t)V;
     float* EPo = R + 4 * ((size_t)V + (size_t)F);
-    launch_g<k_c0_faces_g<QUAD, LAK, CAP>>(grid_for(F), kBlock, str, L.ptr, L.ids, F, N, V, L.verts, FPo, s.cface, s.nav, s.cnt2,
+    launch_g<k_c0_faces_g<QUAD, LAK, CAP>>(grid_for(F), kBlock, str, L.ptr, L.ids, F, N, V, L.verts, FPo, s.cface, L.export_state ? s.nav : nullptr, s.cnt2,
                                            s.rank, s.rec, st);
     lc.after("k_c0_faces");
     const int nt = (int)std::max<int64_t>(1, scan_tiles(V));
@@ -489,7 +489,7 @@ void launch_closed0_t(const Level& L, bool creased, bool comp, Scratch& s, DevSt
         launch_g<k_c0_bucket_g<QUAD>>(grid_for(N), kBlock, str, fc, L.ids, N, F, V, s.sptr, s.rank, s.rec);
         lc.after("k_c0_bucket");
     }
-    const C0Out o{s.xslot, s.xtw, s.xnt, s.eid, s.sc, s.snext, s.sprev, s.sprevc, s.sflag, creased ? 1 : 0};
+    const C0Out o{s.xslot, s.xtw, L.export_state ? s.xnt : nullptr, s.eid, s.sc, s.snext, s.sprev, s.sprevc, s.sflag, creased ? 1 : 0};
     launch_g<k_c0_verts_g<QUAD, LAK, CAP>>(grid_for(V, 128), 128, str, L.ptr, V, E, s.sptr, s.eptr, s.rec, o, L.verts,
                                            FPo, R, comp ? 1 : 0, st);
     lc.after("k_c0_verts");
@@ -816,7 +816,8 @@ void plan_carve(slak_plan* p, Carver& cv)
     p->st = cv.take<DevStatus>(1);
     if (nlev && p->lv[0].closed0) {
         const Level& L0 = p->lv[0];
-        carve_closed0(cv, p->s, L0.N, L0.V, !L0.quad, L0.cap0, !L0.cap0 || p->crease_levels > 0);
+        carve_closed0(cv, p->s, L0.N, L0.V, !L0.quad, L0.cap0, !L0.cap0 || p->crease_levels > 0,
+                      L0.export_state);
     } else {
         carve_scratch(cv, p->s, p->maxN, p->maxV, p->maxE, p->any_poly);
         if (p->exN) carve_export(cv, p->s, p->exN, p->exE);
