@@ -1687,7 +1687,11 @@ size_t batch_plan_groups(slak_batch* b, const std::vector<int64_t>& cand, const 
                          const std::vector<double>& cost, size_t slice, std::vector<size_t>& aoff, cudaStream_t str,
                          int* rc)
 {
-    std::map<std::vector<std::pair<uintptr_t, unsigned>>, std::vector<int64_t>> kinds;
+    std::map<std::vector<std::pair<uintptr_t, unsigned>>, size_t> kind_of;
+    // (kinds in mesh order: a map ordered by the kernels' addresses enqueued the
+    // groups differently with every build; 32 uneven meshes took 570 to 597 us by
+    // the order alone, 580 in mesh order, 597 with the longest group first)
+    std::vector<std::vector<int64_t>> kinds;
     for (int64_t i : cand) {
         slak_plan* p = b->plans[i];
         if (ab[i] > slice) continue;
@@ -1702,12 +1706,14 @@ size_t batch_plan_groups(slak_batch* b, const std::vector<int64_t>& cand, const 
         if (*rc != SLAK_OK) return 0;
         std::vector<std::pair<uintptr_t, unsigned>> key;
         for (const auto& x : r) key.emplace_back(reinterpret_cast<uintptr_t>(x.fn), x.block);
-        kinds[key].push_back(i);
+        const size_t k = kind_of.emplace(key, kinds.size()).first->second;
+        if (k == kinds.size()) kinds.emplace_back();
+        kinds[k].push_back(i);
     }
     std::vector<size_t> gbytes;
-    for (auto& kv : kinds) {
+    for (const auto& kind : kinds) {
         size_t used = slice;
-        for (int64_t i : kv.second) {
+        for (int64_t i : kind) {
             if (used + ab[i] > slice) {
                 b->groups.emplace_back();
                 gbytes.push_back(0);
