@@ -26,7 +26,7 @@
 // Why: these passes move little (about 100 MB at 1 M corners) and are bound by
 // the latency of dependent launches and gathers, so fewer passes is what
 // counts.  Measured on B200, launch by launch: 243,905 polygons (1 M corners)
-// 163 -> 92 us, 400,000 triangles in scattered order (LAK) 250 -> 116 us; whole
+// 163 -> 97 us, 400,000 triangles in scattered order (LAK) 250 -> 119 us; whole
 // plans: 32x32 torus, 3 levels 39.5 -> 26.2 us, 1280 triangles, 4 levels
 // 81.8 -> 55.7 us, the scattered triangles, 1 level 200 -> 107 us.  CAP needs 128
 // bytes per vertex, so it stays with valences up to 8; above that the compact

@@ -273,10 +273,9 @@ __device__ __forceinline__ void for_each_loaded(int n, Load load, Add add)
 
 // ---------------------------------------------------------------- ordering
 // Columns longer than kBigCol slots (and up to kWarpCol) are taken by their
-// whole warp: each lane holds two slots, ranks and loads run in parallel, and
-// the sums run in the fixed order by shuffle (same bits as the single-thread
-// paths, no shared memory).  Shorter columns, and longer ones, stay on one
-// thread.
+// whole warp: ranks and loads run in parallel, and the sums run in the fixed
+// order by shuffle (same bits as the single-thread paths).  Shorter columns, and
+// longer ones, stay on one thread.
 constexpr int kBigCol = 16;
 constexpr int kWarpCol = 64;
 

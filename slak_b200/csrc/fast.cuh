@@ -22,7 +22,12 @@
 //   LAK   edges around edge point e are 4e + {lower end, higher end,
 //         lower face point, higher face point}      [ascending (max, min)]
 //
-// Two kernels per level when P has quad faces, four when P is the polygon
+// These kernels run level 1 of a quad input, every level of an open mesh and the
+// layouts kept for comparison; closed meshes run level 1 of a polygon input
+// (poly1.cuh) and every level from 2 on (grand.cuh) otherwise, with k_g3 from
+// here.
+//
+// Two kernels per level when P has quad faces, four when P is an open polygon
 // input; every output is written exactly once:
 //   k_g1  per quad of C: C's refined quads, face points of C and the next
 //         level's per-corner state; with quad P (4 lanes per face of P) also

@@ -32,9 +32,11 @@
 // registers, 16 warps per SM; one thread per C quad (k_g1, 64 registers, 32
 // warps with three or four each, and warp shuffles for what a thread here
 // holds) was bound by load latency.  Measured on B200, last level of the
-// 512x512 mixed torus: SLAK k_g1 + k_g3 590 + 166 us -> k_pp + k_g3 407 + 52 us
-// (5.7 TB/s of algorithmic bytes, 87% of copy bandwidth), LAK 752 + 125 ->
-// 635 + 50 us; step 1.150 -> 0.780 ms (SLAK), 1.261 -> 1.065 ms (LAK).
+// 512x512 mixed torus: SLAK k_g1 + k_g3 590 + 166 us -> k_pp + k_g3 402 + 52 us
+// (5.7 TB/s of algorithmic bytes, 88% of copy bandwidth), LAK 752 + 125 ->
+// 634 + 50 us; this step alone took the whole call from 1.150 to 0.780 ms (SLAK)
+// and 1.261 to 1.065 ms (LAK).  A cap of 96 registers (20 warps) spills 48-116
+// bytes: 402 -> 472 us, LAK 634 -> 716 us.
 #pragma once
 
 #include "fast.cuh"
