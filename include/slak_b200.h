@@ -304,8 +304,8 @@ int slak_autotune_reset(void);    /* forget the in-process cache (the file is ke
  *    the execution's status SLAK_ERR_BAD_MESH.
  *  - A sharpness that is not finite gives SLAK_ERR_INVALID_ARG.
  *
- * The crease pass runs after each level that has a live crease. It needs four
- * launches, and a mesh without creases pays nothing.
+ * The crease pass runs after each level that has a live crease. It needs one
+ * launch (two more at level 0), and a mesh without creases pays nothing.
  * slak_subdivide_creased is slak_subdivide with creases. It uses no workspace
  * cache.
  */

@@ -304,7 +304,6 @@ void carve_closed0(Carver& cv, Scratch& s, int64_t N, int64_t V, bool poly, bool
     s.sprev = slots ? cv.take<int>(N) : nullptr;
     s.sprevc = slots ? cv.take<int>(N) : nullptr;
     s.sflag = slots ? cv.take<int>(N) : nullptr;
-    s.tmp = slots ? cv.take<int>(scan_tiles(V) + 2) : nullptr;      // the creases' scan
 }
 
 // E > 0: the exported level has a boundary, so its edges' boundary ranks go too
@@ -533,31 +532,19 @@ void launch_creases_t(slak_plan* p, int li, Faces<QUAD> fc, Lc& lc)
         launch_k(k_crease_resolve, grid_for(m), kBlock, str, p->c_pairs, p->c_sharp, (int)m, V0, p->s.sptr, p->s.sc,
                                                           p->s.snext, p->c_mark, p->c_cc[0], p->c_cs[0], p->st);
         lc.after("k_crease_resolve");
-        launch_k(k_crease_vinc<false>, grid_for(V0), kBlock, str, V0, p->s.sptr, p->s.sc, p->s.sprevc, p->s.sflag,
-                                                               SF_BOUT | SF_BIN, p->c_mark, p->c_vcnt, p->c_bnd0,
-                                                               nullptr, nullptr);
-        lc.after("k_crease_vinc");
-        int64_t ns = 0;
-        scan_exclusive(p->c_vcnt, p->c_vptr, V0, p->s.tmp, str, &ns);
-        lc.after("scan(crease vertices)", (int)ns);
-        launch_k(k_crease_vinc<true>, grid_for(V0), kBlock, str, V0, p->s.sptr, p->s.sc, p->s.sprevc, p->s.sflag,
-                                                              SF_BOUT | SF_BIN, p->c_mark, nullptr, nullptr,
-                                                              p->c_vptr, p->c_inc);
+        launch_k(k_crease_vinc, grid_for(V0), kBlock, str, V0, p->s.sptr, p->s.sc, p->s.sprevc, p->s.sflag,
+                 SF_BOUT | SF_BIN, p->c_mark, p->c_vcnt, p->c_vptr, p->c_inc, p->c_bnd0);
         lc.after("k_crease_vinc");
     }
     const bool more = li + 1 < p->crease_levels;
-    launch_k(k_crease_edges<QUAD>, grid_for(n), kBlock, str, fc, L.ids, L.o_ids, L.verts, L.o_verts, p->c_cc[li],
-                                                          p->c_cs[li], (int)n, more ? p->c_cc[li + 1] : nullptr,
-                                                          more ? p->c_cs[li + 1] : nullptr,
-                                                          more ? p->c_ep[li] : nullptr);
-    lc.after("k_crease_edges");
     CreaseEps eps{};
     for (int t = 0; t < li; ++t) eps.epid[t] = p->c_ep[t];
     const int64_t nv = (int64_t)V0 + m * ((1ll << li) - 1);
-    launch_k(k_crease_verts<QUAD>, grid_for(nv), kBlock, str, fc, li, V0, m, L.ids, p->c_cc[li], p->c_cs[li],
-                                                           p->c_vcnt, p->c_vptr, p->c_inc, p->c_bnd0, eps, p->c_vcs, L.verts,
-                                                           L.o_verts);
-    lc.after("k_crease_verts");
+    const unsigned nb = grid_for(n);
+    launch_k(k_crease<QUAD>, nb + grid_for(nv), kBlock, str, fc, li, V0, m, L.ids, L.o_ids, p->c_cc[li], p->c_cs[li],
+             (int)n, more ? p->c_cc[li + 1] : nullptr, more ? p->c_cs[li + 1] : nullptr, more ? p->c_ep[li] : nullptr,
+             p->c_vcnt, p->c_vptr, p->c_inc, p->c_bnd0, eps, p->c_vcs, L.verts, L.o_verts, (int)nb);
+    lc.after("k_crease");
 }
 
 void launch_creases(slak_plan* p, int li, Lc& lc)
@@ -851,8 +838,8 @@ void plan_carve(slak_plan* p, Carver& cv)
         p->c_bnd0 = p->lv[0].B > 0 ? cv.take<unsigned char>(p->lv[0].V) : nullptr;
         p->c_vcs = p->h_vcs.empty() ? nullptr : cv.take<float>(p->lv[0].V);
         p->c_vcnt = cv.take<int>(p->lv[0].V);
-        p->c_vptr = cv.take<int>(p->lv[0].V + 1);
-        p->c_inc = cv.take<int>(2 * m);
+        p->c_vptr = cv.take<int>(p->lv[0].V);
+        p->c_inc = cv.take<int>(p->lv[0].N);
         p->c_cc.assign(p->crease_levels, nullptr);
         p->c_cs.assign(p->crease_levels, nullptr);
         p->c_ep.assign(p->crease_levels, nullptr);
