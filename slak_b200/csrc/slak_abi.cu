@@ -266,8 +266,8 @@ namespace {
 // scratch for one level of at most N corners, V vertices, E edges
 void carve_scratch(Carver& cv, Scratch& s, int64_t N, int64_t V, int64_t E, bool poly)
 {
+    s.cnt = cv.take<int>(V);                                 // (these two start at zero)
     s.cface = poly ? cv.take<int>(N) : nullptr;
-    s.cnt = cv.take<int>(V);
     s.sptr = cv.take<int>(V + 1);
     s.sc = cv.take<int>(N);
     s.snext = cv.take<int>(N);
@@ -337,13 +337,14 @@ int slak::scan_launch(const int* in, int* out, int64_t n, int* tmp, cudaStream_t
 namespace {
 
 // Topology of a level up to the edge-offset scan (needs no output buffers).
-void launch_topology_a(const Level& L, int li, int scheme, Scratch& s, DevStatus* st, Lc& lc)
+// `zeroed`: the counts (and a polygon level's face map) already are.
+void launch_topology_a(const Level& L, int li, int scheme, Scratch& s, DevStatus* st, Lc& lc, bool zeroed = false)
 {
     const int F = (int)L.F, V = (int)L.V, N = (int)L.N;
     cudaStream_t str = lc.s;
-    zero_async(s.cnt, sizeof(int) * (size_t)V, str);
+    if (!zeroed) zero_async(s.cnt, sizeof(int) * (size_t)V, str);
     if (!L.quad) {
-        zero_async(s.cface, sizeof(int) * (size_t)N, str);
+        if (!zeroed) zero_async(s.cface, sizeof(int) * (size_t)N, str);
         launch_g<k_face_map_valence_g>(grid_for(F), kBlock, str, L.ptr, L.ids, F, N, V, s.cface, s.cnt, st);
         lc.after("k_face_map_valence");
     } else {
@@ -576,8 +577,14 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
     // a closed level 0's counts follow the status word in a plan's own arena
     const bool c0 = !p->lv.empty() && p->lv[0].closed0;
     const size_t stb = align_up(sizeof(DevStatus)), cnb = c0 ? sizeof(u64) * (size_t)p->lv[0].V : 0;
+    bool zeroed = false;            // a general level 0's counts and face map follow it likewise
     if (c0 && reinterpret_cast<char*>(p->s.cnt2) == reinterpret_cast<char*>(p->st) + stb) {
         zero_async(p->st, stb + cnb, str);
+    } else if (!c0 && !p->lv.empty() && reinterpret_cast<char*>(p->s.cnt) == reinterpret_cast<char*>(p->st) + stb) {
+        const Level& L0 = p->lv[0];
+        const char* end = p->s.cface ? reinterpret_cast<char*>(p->s.cface + L0.N) : reinterpret_cast<char*>(p->s.cnt + L0.V);
+        zero_async(p->st, (size_t)(end - reinterpret_cast<char*>(p->st)), str);
+        zeroed = true;
     } else {
         zero_async(p->st, sizeof(DevStatus), str);
         if (c0) zero_async(p->s.cnt2, cnb, str);
@@ -599,7 +606,7 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
             if ((int)li < p->crease_levels) launch_creases(p, (int)li, lc);
             continue;
         }
-        launch_topology_a(L, (int)li, p->scheme, p->s, p->st, lc);
+        launch_topology_a(L, (int)li, p->scheme, p->s, p->st, lc, zeroed && li == 0);
         // slot / twin of an exported SLAK state come from k_vsort / k_edges, t from k_refine
         if (L.quad) launch_rest<true>(L, (int)li, p->scheme, comp, p->s, p->st, lc);
         else launch_rest<false>(L, (int)li, p->scheme, comp, p->s, p->st, lc);
