@@ -1170,7 +1170,8 @@ static int plan_create_impl(const slak_mesh* cm, int target_level, int scheme, i
         std::copy(ws->side, ws->side + 2, p->side);
         std::copy(ws->cev, ws->cev + 4, p->cev);
         p->side_owned = false;
-    } else if (rc == SLAK_OK) {
+    } else if (rc == SLAK_OK && !p->lv[0].closed0) {
+        // (a closed mesh's levels have no kernels to run side by side; two streams take 220 us to make)
         for (int k = 0; k < 2 && ce == cudaSuccess; ++k) ce = cudaStreamCreateWithFlags(&p->side[k], cudaStreamNonBlocking);
         for (int k = 0; k < 4 && ce == cudaSuccess; ++k) ce = cudaEventCreateWithFlags(&p->cev[k], cudaEventDisableTiming);
         if (ce != cudaSuccess) rc = cuda_status(ce);
