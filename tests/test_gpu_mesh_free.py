@@ -1,0 +1,64 @@
+"""slak_mesh_free of a one-shot call's result: it waits for whatever still uses
+the arrays, on any stream, as cudaFree does; and it may be called while another
+thread captures a graph in thread-local mode, as cudaFree may, without failing
+and without invalidating that capture."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from slak_b200 import _abi, api, meshgen
+from slak_b200.mesh import SLAK
+
+pytestmark = pytest.mark.gpu
+
+
+def _call(dm, levels=2):
+    cin, c = dm.as_c(), _abi.SlakMesh()
+    _abi.check(_abi.lib().slak_subdivide(ctypes.byref(cin), ctypes.byref(c), levels, SLAK, None), "slak_subdivide")
+    return c
+
+
+def _free(c):
+    return _abi.lib().slak_mesh_free(ctypes.byref(c))
+
+
+def test_free_waits_for_work_on_other_streams():
+    dm = api.DeviceMesh.from_host(meshgen.torus(16, 12, seed=1))
+    s = torch.cuda.Stream()
+    for _ in range(3):                              # the first wait and later ones
+        c = _call(dm)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(10_000_000)           # about 5 ms
+        assert not s.query()
+        assert _free(c) == _abi.SLAK_OK
+        assert s.query()
+
+
+def test_free_beside_another_threads_capture():
+    m = meshgen.torus(16, 12, seed=1)
+    dm = api.DeviceMesh.from_host(m)
+    results = [_call(dm) for _ in range(2)]
+    torch.cuda.synchronize()
+    x, rc = torch.zeros(16, device="cuda"), []
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        x += 1
+        t = threading.Thread(target=lambda: rc.extend(_free(c) for c in results))
+        t.start()
+        t.join()
+        x += 1
+    g.replay()
+    torch.cuda.synchronize()
+    assert rc == [_abi.SLAK_OK] * 2
+    assert x.tolist() == [2.0] * 16
+    # the freed arrays serve the next call
+    out = api.DeviceMesh()
+    api.CatmullClark.subdivideIteratively(dm, out, 2)
+    ref = oracle.subdivide(m, 2, SLAK)
+    assert np.array_equal(out.ids.cpu().numpy(), ref.ids)
+    assert np.array_equal(out.verts.cpu().numpy().view(np.uint32), ref.verts.reshape(-1).view(np.uint32))
