@@ -85,7 +85,8 @@ const char* slak_last_error_detail(void);
  * per-device workspace that is kept for the next call (the reference
  * allocates and frees them inside every call); a call made while another
  * holds the workspace allocates its own.  Output arrays that came back through
- * slak_mesh_free are kept too, at most 1 GiB per device, and handed out again.
+ * slak_mesh_free are kept too, at most 1 GiB per device, and handed out again;
+ * they give way to any allocation of this library that would not fit beside them.
  * SLAK_WORKSPACE_CACHE=0 in the environment turns both off.
  */
 int slak_subdivide(const slak_mesh* cmesh, slak_mesh* rmesh, int target_level, int scheme,

@@ -71,7 +71,8 @@ struct Carver {
 // host (at any size up to 64 MiB), five to ten times the refinement of a small
 // mesh, so the arrays that slak_mesh_free gets back are kept, idle, for later
 // calls on the same device: at most kOutCacheBytes per device, returned by
-// slak_workspace_release and before an allocation of this library fails;
+// slak_workspace_release, before a device allocation of this library fails
+// (device_malloc, all of them) and before they limit a batch's memory;
 // SLAK_WORKSPACE_CACHE=0 turns it off.  Only arrays these calls allocated are
 // kept; one the caller freed with cudaFree just leaves the table (its entry is
 // checked against the driver's allocation before it is believed).
@@ -123,6 +124,15 @@ cudaError_t device_malloc(void** p, size_t bytes)
         cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
+    return e;
+}
+
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes)
+{
+    void* q = nullptr;
+    const cudaError_t e = device_malloc(&q, bytes);
+    if (e == cudaSuccess) *p = static_cast<T*>(q);
     return e;
 }
 
@@ -714,7 +724,7 @@ int probe_level0(slak_plan* p, Level& L0, cudaStream_t str, void* given = nullpt
     void* mem = given;
     cudaError_t e = cudaSuccess;
     if (!given) {
-        e = cudaMalloc(&mem, probe_bytes(L0));
+        e = device_malloc(&mem, probe_bytes(L0));
         if (e != cudaSuccess) return cuda_status(e);
     }
     Carver cv((char*)mem);
@@ -1240,7 +1250,7 @@ static int plan_create_impl(const slak_mesh* cm, int target_level, int scheme, i
     slak_mesh o = plan_output_shape(p);
     // (a one-shot call's come from the idle ones)
     const auto out = [&](auto** q, size_t bytes) {
-        if (ce == cudaSuccess) ce = ws ? out_malloc(q, bytes) : device_malloc(reinterpret_cast<void**>(q), bytes);
+        if (ce == cudaSuccess) ce = ws ? out_malloc(q, bytes) : device_malloc(q, bytes);
     };
     out(&o.ids, sizeof(int) * (size_t)o.nnz);
     out(&o.verts, sizeof(float) * 4 * (size_t)o.nverts);
@@ -1835,7 +1845,7 @@ int batch_upload_groups(slak_batch* b, cudaStream_t str)
             st.grid = (unsigned)tot;
         }
     }
-    cudaError_t ce = cudaMalloc(&b->gmem, off);
+    cudaError_t ce = device_malloc(&b->gmem, off);
     if (ce == cudaSuccess) ce = cudaMemcpy(b->gmem, hb.data(), off, cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) return cuda_status(ce);
     const int ns = *std::max_element(b->gstream_of.begin(), b->gstream_of.end()) + 1;
@@ -1899,7 +1909,7 @@ static int batch_create_impl(const slak_mesh* meshes, const int* levels, int64_t
         carve_scratch(dry, sc, maxN, maxV, 1, any_poly);
         DevStatus* st = dry.take<DevStatus>(1);
         void* mem = nullptr;
-        ce = cudaMalloc(&mem, dry.off);
+        ce = device_malloc(&mem, dry.off);
         if (ce != cudaSuccess) rc = cuda_status(ce);
         else {
             Carver cv((char*)mem);
@@ -1954,13 +1964,20 @@ static int batch_create_impl(const slak_mesh* meshes, const int* levels, int64_t
         cost[i] = batch_cost_us(p);
     }
     if (rc == SLAK_OK) {
-        size_t freeb = 0, totalb = 0;
-        cudaMemGetInfo(&freeb, &totalb);
-        const size_t margin = size_t(2) << 30;
-        if (total_out + margin > freeb) { g_detail = "batch outputs exceed device memory"; rc = SLAK_ERR_OOM; }
-        size_t budget = rc == SLAK_OK ? (freeb - total_out - margin) * 3 / 4 : 0;
         size_t cap = size_t(24) << 30;
         if (const char* wb = std::getenv("SLAK_BATCH_WAVE_BYTES")) cap = (size_t)std::strtoull(wb, nullptr, 10);
+        const size_t margin = size_t(2) << 30;
+        size_t freeb = 0, totalb = 0;
+        cudaMemGetInfo(&freeb, &totalb);
+        // idle output arrays are given back before they refuse the batch or limit
+        // its scratch (`scratch`: what it has use for, by the rules below)
+        size_t most = 0, sum = 0;
+        for (size_t x : ab) { most = std::max(most, x); sum += x; }
+        const size_t scratch = std::max(most, std::min(cap, 2 * kGroupStreams * sum));
+        const int dev = current_device();
+        if (dev >= 0 && total_out + margin + scratch / 3 * 4 + 4 > freeb && out_trim(dev)) cudaMemGetInfo(&freeb, &totalb);
+        if (total_out + margin > freeb) { g_detail = "batch outputs exceed device memory"; rc = SLAK_ERR_OOM; }
+        size_t budget = rc == SLAK_OK ? (freeb - total_out - margin) * 3 / 4 : 0;
         if (budget > cap) budget = cap;
         // small meshes run in groups (kinds of identical launch sequences cut
         // into groups of at most `slice` bytes of scratch); the groups' part
@@ -2040,9 +2057,9 @@ static int batch_create_impl(const slak_mesh* meshes, const int* levels, int64_t
         b->arena_bytes = goff + gbytes;
     }
     if (rc == SLAK_OK && total_out) {
-        if (!b->per_mesh_out) ce = cudaMalloc(&b->out_mem, total_out);
-        if (ce == cudaSuccess && b->arena_bytes) ce = cudaMalloc(&b->arena, b->arena_bytes);
-        if (ce == cudaSuccess) ce = cudaMalloc(&b->d_st, sizeof(DevStatus) * (size_t)count);
+        if (!b->per_mesh_out) ce = device_malloc(&b->out_mem, total_out);
+        if (ce == cudaSuccess && b->arena_bytes) ce = device_malloc(&b->arena, b->arena_bytes);
+        if (ce == cudaSuccess) ce = device_malloc(&b->d_st, sizeof(DevStatus) * (size_t)count);
         if (ce != cudaSuccess) rc = cuda_status(ce);
     }
     if (rc == SLAK_OK && b->per_mesh_out) {
