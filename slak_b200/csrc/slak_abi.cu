@@ -80,8 +80,9 @@ constexpr size_t kOutCacheBytes = size_t(1) << 30;
 constexpr int kWsMaxDevices = 64;
 
 struct OutBlock {
-    size_t bytes;
+    size_t bytes;       // asked for
     int dev;
+    size_t range;       // the driver's size of the allocation
 };
 std::mutex g_out_mu;
 std::map<void*, OutBlock> g_out_live;                                   // handed out
@@ -101,6 +102,23 @@ int current_device()
     return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kWsMaxDevices ? dev : -1;
 }
 
+// the size of the allocation that starts at p, 0 if none does
+size_t allocation_size(void* p)
+{
+    static const auto range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr)>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (range == nullptr || range(&base, &size, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return 0;
+    return base == reinterpret_cast<CUdeviceptr>(p) ? size : 0;
+}
+
 // frees the device's idle blocks; true if there were any
 bool out_trim(int dev)
 {
@@ -115,7 +133,8 @@ bool out_trim(int dev)
     return !v.empty();
 }
 
-// cudaMalloc that gives the idle blocks back before it fails
+// cudaMalloc that gives the idle blocks back before it fails.  An entry of the
+// table under the new address is of an array that the caller freed with cudaFree.
 cudaError_t device_malloc(void** p, size_t bytes)
 {
     cudaError_t e = cudaMalloc(p, bytes);
@@ -123,6 +142,10 @@ cudaError_t device_malloc(void** p, size_t bytes)
     if (dev >= 0 && out_trim(dev)) {
         cudaGetLastError();
         e = cudaMalloc(p, bytes);
+    }
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(g_out_mu);
+        g_out_live.erase(*p);
     }
     return e;
 }
@@ -146,15 +169,16 @@ cudaError_t out_malloc(void** p, size_t bytes)
         if (it != g_out_idle[dev].end() && it->first / 2 <= std::max(bytes, size_t(1) << 16)) {
             *p = it->second;
             g_out_idle_bytes[dev] -= it->first;
-            g_out_live[*p] = OutBlock{it->first, dev};
+            g_out_live[*p] = OutBlock{it->first, dev, allocation_size(*p)};
             g_out_idle[dev].erase(it);
             return cudaSuccess;
         }
     }
     const cudaError_t e = device_malloc(p, bytes);
     if (e == cudaSuccess && dev >= 0) {
+        const size_t range = allocation_size(*p);
         std::lock_guard<std::mutex> lk(g_out_mu);
-        g_out_live[*p] = OutBlock{bytes, dev};
+        g_out_live[*p] = OutBlock{bytes, dev, range};
     }
     return e;
 }
@@ -222,27 +246,16 @@ bool out_known(std::initializer_list<void*> v)
 
 // Keeps `p` idle instead of freeing it; false if it is not one of these
 // blocks (or no longer: the caller freed it and the address was allocated
-// again) or does not fit.  The caller waited for the device (device_wait).
+// again, with another size) or does not fit.  The caller waited for the device
+// (device_wait).
 bool out_keep(void* p, int dev)
 {
-    static const auto range = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr)>(f);
-    }();
     std::lock_guard<std::mutex> lk(g_out_mu);
     auto it = g_out_live.find(p);
     if (it == g_out_live.end()) return false;
     const OutBlock b = it->second;
     g_out_live.erase(it);
-    CUdeviceptr base = 0;
-    size_t size = 0;
-    if (b.dev != dev || range == nullptr || range(&base, &size, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS ||
-        base != reinterpret_cast<CUdeviceptr>(p) || size < b.bytes)
-        return false;
+    if (b.dev != dev || b.range == 0 || allocation_size(p) != b.range) return false;
     if (g_out_idle_bytes[dev] + b.bytes > kOutCacheBytes) return false;
     g_out_idle[dev].emplace(b.bytes, p);
     g_out_idle_bytes[dev] += b.bytes;

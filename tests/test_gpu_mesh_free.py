@@ -62,3 +62,45 @@ def test_free_beside_another_threads_capture():
     ref = oracle.subdivide(m, 2, SLAK)
     assert np.array_equal(out.ids.cpu().numpy(), ref.ids)
     assert np.array_equal(out.verts.cpu().numpy().view(np.uint32), ref.verts.reshape(-1).view(np.uint32))
+
+
+def _cudart():
+    import glob
+    import os
+    import nvidia.cuda_runtime
+    return ctypes.CDLL(glob.glob(os.path.join(list(nvidia.cuda_runtime.__path__)[0], "lib", "libcudart.so*"))[0])
+
+
+def _allocation_size(p):
+    base, size = ctypes.c_uint64(), ctypes.c_size_t()
+    assert ctypes.CDLL("libcuda.so.1").cuMemGetAddressRange_v2(ctypes.byref(base), ctypes.byref(size),
+                                                               ctypes.c_uint64(p)) == 0
+    assert base.value == p
+    return size.value
+
+
+def test_an_address_that_was_freed_and_allocated_larger():
+    """A result freed with cudaFree whose address comes back as another, larger
+    array: slak_mesh_free of that one must not keep it under the old size."""
+    lib, cudart = _abi.lib(), _cudart()
+    dm = api.DeviceMesh.from_host(meshgen.torus(16, 12, seed=1))
+    assert lib.slak_workspace_release() == _abi.SLAK_OK
+    c = _call(dm)
+    size, want = 4 * c.nnz, 4 * c.nnz + 32768       # (ids and verts are 48 KiB each, one behind the other)
+    old = c.ids
+    for p in (c.ids, c.verts):
+        assert cudart.cudaFree(ctypes.c_void_p(p)) == 0
+    again = []
+    for _ in range(16):                             # the driver's first fit: usually the first
+        p = ctypes.c_void_p()
+        assert cudart.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(want)) == 0
+        again.append(p.value)
+        if p.value == old:
+            break
+    for p in again:
+        m = _abi.SlakMesh()
+        m.ids = p
+        assert _free(m) == _abi.SLAK_OK
+    n = _call(dm)
+    assert _allocation_size(n.ids) == size and _allocation_size(n.verts) == 16 * n.nverts
+    assert _free(n) == _abi.SLAK_OK
