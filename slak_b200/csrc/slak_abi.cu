@@ -21,6 +21,7 @@
 #include <cmath>
 #include <initializer_list>
 #include <map>
+#include <set>
 #include <type_traits>
 
 #include "plan.cuh"
@@ -88,6 +89,7 @@ std::mutex g_out_mu;
 std::map<void*, OutBlock> g_out_live;                                   // handed out
 std::multimap<size_t, void*> g_out_idle[kWsMaxDevices];                 // by size
 size_t g_out_idle_bytes[kWsMaxDevices] = {};
+std::set<void*> g_out_idle_set;                                         // every device's idle blocks
 void* g_out_token[kWsMaxDevices] = {};                                  // see device_wait
 
 bool workspace_cached()
@@ -125,7 +127,10 @@ bool out_trim(int dev)
     std::vector<void*> v;
     {
         std::lock_guard<std::mutex> lk(g_out_mu);
-        for (const auto& e : g_out_idle[dev]) v.push_back(e.second);
+        for (const auto& e : g_out_idle[dev]) {
+            v.push_back(e.second);
+            g_out_idle_set.erase(e.second);
+        }
         g_out_idle[dev].clear();
         g_out_idle_bytes[dev] = 0;
     }
@@ -166,11 +171,15 @@ cudaError_t out_malloc(void** p, size_t bytes)
     if (dev >= 0) {
         std::lock_guard<std::mutex> lk(g_out_mu);
         auto it = g_out_idle[dev].lower_bound(bytes);
-        if (it != g_out_idle[dev].end() && it->first / 2 <= std::max(bytes, size_t(1) << 16)) {
-            *p = it->second;
-            g_out_idle_bytes[dev] -= it->first;
-            g_out_live[*p] = OutBlock{it->first, dev, allocation_size(*p)};
-            g_out_idle[dev].erase(it);
+        while (it != g_out_idle[dev].end() && it->first / 2 <= std::max(bytes, size_t(1) << 16)) {
+            void* const q = it->second;
+            const size_t size = it->first, range = allocation_size(q);
+            it = g_out_idle[dev].erase(it);
+            g_out_idle_bytes[dev] -= size;
+            g_out_idle_set.erase(q);
+            if (range < size) continue;             // freed behind the table's back
+            g_out_live[q] = OutBlock{size, dev, range};
+            *p = q;
             return cudaSuccess;
         }
     }
@@ -225,12 +234,14 @@ void token_release(int dev)
     if (t) cudaFree(t);
 }
 
-// cudaFree of an array that may be in the table
+// cudaFree of an array that may be in the table; an idle block is not the
+// caller's any more (a second free of it), which is cudaFree's error for such
 cudaError_t out_free(void* p)
 {
     {
         std::lock_guard<std::mutex> lk(g_out_mu);
         g_out_live.erase(p);
+        if (g_out_idle_set.count(p)) return cudaErrorInvalidValue;
     }
     return cudaFree(p);
 }
@@ -258,6 +269,7 @@ bool out_keep(void* p, int dev)
     if (b.dev != dev || b.range == 0 || allocation_size(p) != b.range) return false;
     if (g_out_idle_bytes[dev] + b.bytes > kOutCacheBytes) return false;
     g_out_idle[dev].emplace(b.bytes, p);
+    g_out_idle_set.insert(p);
     g_out_idle_bytes[dev] += b.bytes;
     return true;
 }

@@ -104,3 +104,23 @@ def test_an_address_that_was_freed_and_allocated_larger():
     n = _call(dm)
     assert _allocation_size(n.ids) == size and _allocation_size(n.verts) == 16 * n.nverts
     assert _free(n) == _abi.SLAK_OK
+
+
+def test_a_second_free_is_an_error_and_harms_no_later_result():
+    """A copied descriptor freed twice: the second free is refused (as cudaFree
+    would), and the arrays kept by the first stay good for later calls."""
+    m = meshgen.torus(16, 12, seed=1)
+    dm, ref = api.DeviceMesh.from_host(m), oracle.subdivide(m, 2, SLAK)
+    c = _call(dm)
+    copy = _abi.SlakMesh.from_buffer_copy(c)
+    assert _free(c) == _abi.SLAK_OK
+    assert _free(copy) == 2                         # SLAK_ERR_CUDA
+    outs = []
+    for _ in range(2):
+        out = api.DeviceMesh()
+        api.CatmullClark.subdivideIteratively(dm, out, 2)
+        outs.append(out)
+    assert outs[0].ids.data_ptr() != outs[1].ids.data_ptr()
+    for out in outs:
+        assert np.array_equal(out.ids.cpu().numpy(), ref.ids)
+        assert np.array_equal(out.verts.cpu().numpy().view(np.uint32), ref.verts.reshape(-1).view(np.uint32))
