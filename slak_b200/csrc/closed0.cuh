@@ -65,6 +65,44 @@ __device__ __forceinline__ void c0_corner(int c, int f, int v, int w, int u, boo
     }
 }
 
+// A face of n > kBigCol corners from b on by its warp: corners over the lanes,
+// the sum of its positions in corner order, one component per lane.  One thread
+// waits for each corner's atomic in turn (its result is the corner's place).
+// Level 0 of a prism on B200, by its caps' corners: 17 25 -> 19 us, 33 33 -> 19,
+// 64 46 -> 19, 256 153 -> 36, 1000 468 -> 109 (the general level 30, 32, 36, 68 and
+// 188); 2,000 prisms of 24 40 -> 33.  16 corners in turn take 21 us.
+template <bool LAK, bool CAP>
+__device__ __forceinline__ void c0_long_face(const int* __restrict__ ids, int f, int b, int n, int V,
+                                          const float* __restrict__ P, float* __restrict__ FP, int* __restrict__ cface,
+                                          unsigned* __restrict__ nav, unsigned long long* __restrict__ cnt,
+                                          int* __restrict__ rank, int4* __restrict__ rec, DevStatus* st)
+{
+    const int lane = threadIdx.x & 31, c4 = term_comp();
+    for (int k = lane; k < n; k += 32) {
+        const int c = b + k;
+        const int v = __ldg(ids + c), w = __ldg(ids + (k + 1 < n ? c + 1 : b)), u = __ldg(ids + (k ? c - 1 : b + n - 1));
+        cface[c] = f;
+        if (nav != nullptr) nav[c] = n <= 0xffff ? (unsigned)k | ((unsigned)(n - 1 - k) << 16) : kNavFar;
+        c0_corner<LAK, CAP>(c, f, v, w, u, k == 0, V, cnt, rank, rec, st);
+    }
+    float acc = 0.0f;
+    for (int k0 = 0; k0 < n; k0 += 64) {
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = k0 + 8 * j + term_slot();
+            x[j] = 0.0f;
+            if (k < n) {
+                const int v = __ldg(ids + b + k);
+                x[j] = ldg1(P, (unsigned)v < (unsigned)V ? v : 0, c4);
+            }
+        }
+        each_term(x, n - k0, [&](float t) { acc = __fadd_rn(acc, t); });
+    }
+    const float y = LAK ? __fadd_rn(div1(acc, (float)n), 0.0f) : __fmul_rn(acc, __fdiv_rn(1.0f, (float)n));
+    if (lane < 4) FP[4 * (int64_t)f + lane] = y;
+}
+
 template <bool QUAD, bool LAK, bool CAP>
 __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* __restrict__ ptr,
                                                 const int* __restrict__ ids, int F, int N, int V,
@@ -74,10 +112,9 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
                                                 int* __restrict__ rank, int4* __restrict__ rec, DevStatus* st)
 {
     const int f = bx_ * kBlock + threadIdx.x;
-    if (!QUAD && f == 0 && (ptr[0] != 0 || ptr[F] != N)) set_error(st, 4, -1);
-    if (f >= F) return;
     const auto pos = [&](int v) { return ldg4(P, (unsigned)v < (unsigned)V ? v : 0); };
     if constexpr (QUAD) {
+        if (f >= F) return;
         const int4 q = __ldg(reinterpret_cast<const int4*>(ids) + f);
         const float4 a = pos(q.x), b = pos(q.y), c = pos(q.z), e = pos(q.w);
         c0_corner<LAK, CAP>(4 * f + 0, f, q.x, q.y, q.w, true, V, cnt, rank, rec, st);
@@ -87,10 +124,14 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
         if (!LAK) st4(FP, f, f4_mul(f4_add(f4_add(a, c), f4_add(b, e)), 0.25f));
         else st4(FP, f, f4_div_z(f4_add(f4_add(f4_add(f4_add(f4_zero(), a), b), c), e), 4.0f));
     } else {
-        const int b = ptr[f], e = ptr[f + 1], n = e - b;
-        if (b < 0 || e > N || n < 3) { set_error(st, 4, f); return; }
+        if (f == 0 && (ptr[0] != 0 || ptr[F] != N)) set_error(st, 4, -1);
+        int b = 0, e = 0;
+        if (f < F) { b = ptr[f]; e = ptr[f + 1]; }
+        const int n = e - b;
+        const bool ok = b >= 0 && e <= N && n >= 3;
+        if (f < F && !ok) set_error(st, 4, f);
         float4 acc = f4_zero();
-        if (n <= 8) {                   // every id and position in flight at once
+        if (ok && n <= 8) {                   // every id and position in flight at once
             int v[8];
             float4 p[8];
 #pragma unroll
@@ -113,7 +154,7 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
 #pragma unroll
             for (int k = 0; k < 8; ++k)
                 if (k < n) acc = f4_add(acc, p[k]);
-        } else {
+        } else if (ok && n <= kBigCol) {
             int u = __ldg(ids + e - 1), v = __ldg(ids + b);
             for (int c = b; c < e; ++c) {
                 const int w = __ldg(ids + (c + 1 < e ? c + 1 : b));
@@ -125,7 +166,12 @@ __device__ __forceinline__ void k_c0_faces_body(const unsigned bx_, const int* _
                 v = w;
             }
         }
-        st4(FP, f, LAK ? f4_div_z(acc, (float)n) : f4_mul(acc, __fdiv_rn(1.0f, (float)n)));
+        if (ok && n <= kBigCol) st4(FP, f, LAK ? f4_div_z(acc, (float)n) : f4_mul(acc, __fdiv_rn(1.0f, (float)n)));
+        // a long face by its warp: one thread would wait for each corner's atomic in turn
+        for_each_big<kBlock>(ok && n > kBigCol, false, [&](int i) {
+            const int g = bx_ * kBlock + i, gb = ptr[g];
+            c0_long_face<LAK, CAP>(ids, g, gb, ptr[g + 1] - gb, V, P, FP, cface, nav, cnt, rank, rec, st);
+        });
     }
 }
 template <bool QUAD, bool LAK, bool CAP>
