@@ -653,13 +653,16 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
         lc.recs = &p->recs;
         cudaEventRecord(p->ev[0], str);
     }
-    // a closed level 0's counts follow the status word in a plan's own arena
+    // a closed level 0's counts follow the status word in a plan's own arena; a
+    // general level 0's, with the face map behind them, likewise, unless a larger
+    // general level's counts lie between them (SLAK_PLAN_GENERAL)
     const bool c0 = !p->lv.empty() && p->lv[0].closed0;
     const size_t stb = align_up(sizeof(DevStatus)), cnb = c0 ? sizeof(u64) * (size_t)p->lv[0].V : 0;
-    bool zeroed = false;            // a general level 0's counts and face map follow it likewise
+    const bool g0 = !c0 && !p->lv.empty() && p->maxV == p->lv[0].V;
+    bool zeroed = false;
     if (c0 && reinterpret_cast<char*>(p->s.cnt2) == reinterpret_cast<char*>(p->st) + stb) {
         zero_async(p->st, stb + cnb, str);
-    } else if (!c0 && !p->lv.empty() && reinterpret_cast<char*>(p->s.cnt) == reinterpret_cast<char*>(p->st) + stb) {
+    } else if (g0 && reinterpret_cast<char*>(p->s.cnt) == reinterpret_cast<char*>(p->st) + stb) {
         const Level& L0 = p->lv[0];
         const char* end = p->s.cface ? reinterpret_cast<char*>(p->s.cface + L0.N) : reinterpret_cast<char*>(p->s.cnt + L0.V);
         zero_async(p->st, (size_t)(end - reinterpret_cast<char*>(p->st)), str);
