@@ -261,11 +261,16 @@ static void launch_p1_t(const Level& Pl, const Level& L, Faces<false> pf, bool c
     const int64_t g3 = 16 * Pl.V + (LAK ? 0 : 16 * L.F);
     lc.after("k_p1", 1, 4 * L.N + 16 * L.V + (L.skip_ids ? 0 : 16 * L.N) + 16 * L.Vo - g3 +
                             (optr ? 4 * (L.N + 1) + 16 * L.N : 0));
-    with_block(L.bs[2], [&](auto b) {
-        constexpr int BS = decltype(b)::value;
-        launch_g<k_g3_g<LAK, STATE, BS>>(grid_for(Pl.V + 1, BS), BS, lc.s, d, L.verts, L.in_state, L.out_state, L.slots,
-                                         L.o_verts, mode, (int)Pl.V, nullptr, 0);
-    });
+    if (L.bulk3) {
+        launch_g<k_g3_bulk_g<LAK, STATE>>(grid_for(Pl.V + 1, kBulkBlock), kBulkBlock, lc.s, d, L.verts, L.in_state,
+                                          L.out_state, L.slots, L.o_verts, comp ? 1 : 0, (int)Pl.V, L.st, L.bulk_polls);
+    } else {
+        with_block(L.bs[2], [&](auto b) {
+            constexpr int BS = decltype(b)::value;
+            launch_g<k_g3_g<LAK, STATE, BS>>(grid_for(Pl.V + 1, BS), BS, lc.s, d, L.verts, L.in_state, L.out_state, L.slots,
+                                             L.o_verts, mode, (int)Pl.V, nullptr, 0);
+        });
+    }
     lc.after("k_g3", 1, g3);
 }
 
