@@ -239,8 +239,10 @@ typedef struct slak_kernel_timing {
 typedef struct slak_tuning {
     int32_t state;              /* -1 not a fast level, 0 default, 1 measured by this plan,
                                    2 taken from the tuning cache                         */
-    int32_t block[3];           /* block size of k_g1, k_g2, k_g3                          */
-    float ms[3][3];             /* state 1: median ms of each kernel at block 128/256/512  */
+    int32_t block[3];           /* 128, 256 or 512 each.  [0]: block size of k_g1 (k_p1: twice
+                                   its threads, k_pp: four times), [1]: block size of k_g2
+                                   (k_p1: its register cap), [2]: block size of k_g3     */
+    float ms[3][3];             /* state 1: median ms of the kernel at each of the three   */
     char key[64];               /* tuning-cache key                                        */
 } slak_tuning;
 
@@ -268,13 +270,14 @@ int slak_plan_destroy(slak_plan* plan);
 
 /*
  * Autotuner (no counterpart in the reference, whose launch shapes are fixed).
- * The block sizes of the three closed-form kernels of every fast level are
- * chosen by measurement, keyed on the scheme, the parent level's face type,
- * whether the level feeds another fast level, log2 of the level's quads and
- * the input's valence histogram (largest valence; share of valence 4).  Every
+ * The launch shapes (slak_tuning.block) of every fast level are chosen by
+ * measurement, keyed on the scheme, the kernels that run (by the face type of
+ * the level's parent or grandparent), whether the level feeds another fast
+ * level, log2 of the level's quads and the input's valence histogram (largest
+ * valence; share of valence 4).  Every
  * plan and batch applies cached choices; with SLAK_PLAN_AUTOTUNE, creation also
- * measures the keys not yet cached (block 128 / 256 / 512 per kernel, median of
- * three executions).  The cache lives in the process; with SLAK_TUNE_FILE set
+ * measures the keys not yet cached (128 / 256 / 512 for each, median of three
+ * executions).  The cache lives in the process; with SLAK_TUNE_FILE set
  * in the environment it is also loaded from and saved to that file.
  */
 int slak_plan_tuning(const slak_plan* plan, int level, slak_tuning* out);

@@ -1041,13 +1041,16 @@ cudaError_t workspace_reserve(Workspace* w, size_t bytes)
 }  // namespace
 
 // ------------------------------------------------------------------ autotuner
-// The block sizes of k_g1 / k_g2 / k_g3 of every fast level are chosen by
-// measurement.  The key is what sets them: the scheme, the parent's face type,
-// whether the level writes the next level's state, the level's size (log2 of
-// its quads) and the input's valence histogram (largest valence class; share
-// of valence-4 vertices).  Choices are cached per process and, with
-// SLAK_TUNE_FILE set, in that text file (a key and three block sizes a line).
-// Every plan applies cached choices; SLAK_PLAN_AUTOTUNE measures missing keys.
+// Three choices of every fast level are made by measurement, each among 128, 256
+// and 512: [0] the block size of k_g1 (k_p1 runs half as many threads, k_pp a
+// quarter), [1] the block size of k_g2 (k_p1: its register cap, levels.cu), [2] the
+// block size of k_g3.  The key is what sets them: the scheme, the kernels that run
+// (the parent's or grandparent's face type), whether the level writes the next
+// levels' state, the level's size (log2 of its quads) and the input's valence
+// histogram (largest valence class; share of valence-4 vertices).  Choices are
+// cached per process and, with SLAK_TUNE_FILE set, in that text file (a key and
+// three sizes a line).  Every plan applies cached choices; SLAK_PLAN_AUTOTUNE
+// measures missing keys.
 std::mutex g_tune_mu;
 std::map<std::string, std::array<int, 3>> g_tune;
 bool g_tune_loaded = false;
@@ -1068,10 +1071,12 @@ std::string tune_key(const slak_plan* p, int li)
     const int sclass = share4 < 0.5 ? 0 : share4 < 0.9 ? 50 : 90;
     const int fb = (int)std::floor(std::log2((double)std::max<int64_t>(L.F, 1)));
     char buf[96];
+    // the kernels that run: refined from the grandparent's state (by its face
+    // type), the one-launch level 1 of a closed polygon mesh, the others by parent
+    const char* kind = L.pp ? (p->lv[li - 2].quad ? "ppquad" : "pppoly")
+                     : L.gq ? "gquad" : P.quad ? "quad" : P.B > 0 ? "poly" : "poly1";
     std::snprintf(buf, sizeof buf, "%s/%s%s/%s/q2^%d/vmax%d/v4_%d", p->scheme == SLAK_SCHEME_LAK ? "lak" : "slak",
-                  L.gq ? "gquad" : P.quad ? "quad" : "poly", P.B > 0 ? "-open" : "",
-                  L.pp ? (L.make_state ? "pp-state" : "pp-last") : L.make_state ? "state" : L.sg ? "last-sg" : "last",
-                  fb, vclass, sclass);
+                  kind, P.B > 0 ? "-open" : "", L.make_state ? "state" : L.sg ? "last-sg" : "last", fb, vclass, sclass);
     return buf;
 }
 
