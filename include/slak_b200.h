@@ -204,7 +204,9 @@ int slak_subdivide_level_noalloc(const slak_mesh* cmesh, slak_mesh* rmesh, int s
  *
  * slak_plan_create reads the input's topology once (one stream sync) to size
  * all levels.  slak_plan_execute re-runs every level from the current
- * contents of cmesh's arrays, which must keep the same topology.  The refined
+ * contents of cmesh's arrays, which must keep the same topology (an execution
+ * that notices another reports SLAK_ERR_BAD_MESH, but what it reads and writes
+ * is not defined then).  The refined
  * mesh stays owned by the plan (slak_plan_output) until slak_plan_release_output
  * hands the arrays to the caller.
  */

@@ -342,15 +342,17 @@ __device__ __forceinline__ void k_c0_bucket_body(const unsigned bx_, Faces<QUAD>
     if (c >= N) return;
     const int v = __ldg(ids + c);
     if ((unsigned)v >= (unsigned)V) return;
-    // (a malformed mesh's corner in a face the first pass rejected has neither
-    // face nor rank of this run: every index is kept in range)
+    // (a plan's mesh keeps its topology; where the caller changed it all the same,
+    // a corner of a face the first pass rejected has neither face nor rank of this
+    // run, and overlapping faces count more than N corners: what is read and written
+    // here stays in range)
     int f, nc, p;
     c0_nav<QUAD>(fc, c, N, F, f, nc, p);
     int w = __ldg(ids + nc), u = __ldg(ids + p);
     if ((unsigned)w >= (unsigned)V) w = v;
     if ((unsigned)u >= (unsigned)V) u = v;
     const int b = __ldg(sptr + v), r = __ldg(rank + c);
-    if ((unsigned)r < (unsigned)(__ldg(sptr + v + 1) - b))
+    if ((unsigned)r < (unsigned)(__ldg(sptr + v + 1) - b) && (unsigned)(b + r) < (unsigned)N)
         rec[b + r] = make_int4(c, p > c ? (int)((unsigned)w | kFirst) : w, u, f);
 }
 template <bool QUAD>
