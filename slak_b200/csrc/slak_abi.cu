@@ -655,14 +655,18 @@ int enqueue_all(slak_plan* p, cudaStream_t str)
     }
     // a closed level 0's counts follow the status word in a plan's own arena; a
     // general level 0's, with the face map behind them, likewise, unless a larger
-    // general level's counts lie between them (SLAK_PLAN_GENERAL)
+    // general level's counts lie between them (SLAK_PLAN_GENERAL).  A recorded
+    // sequence keeps them apart: it must not depend on addresses
     const bool c0 = !p->lv.empty() && p->lv[0].closed0;
     const size_t stb = align_up(sizeof(DevStatus)), cnb = c0 ? sizeof(u64) * (size_t)p->lv[0].V : 0;
     const bool g0 = !c0 && !p->lv.empty() && p->maxV == p->lv[0].V;
     bool zeroed = false;
-    if (c0 && reinterpret_cast<char*>(p->s.cnt2) == reinterpret_cast<char*>(p->st) + stb) {
+    const auto follows = [&](const void* counts) {
+        return !g_record && static_cast<const char*>(counts) == reinterpret_cast<const char*>(p->st) + stb;
+    };
+    if (c0 && follows(p->s.cnt2)) {
         zero_async(p->st, stb + cnb, str);
-    } else if (g0 && reinterpret_cast<char*>(p->s.cnt) == reinterpret_cast<char*>(p->st) + stb) {
+    } else if (g0 && follows(p->s.cnt)) {
         const Level& L0 = p->lv[0];
         const char* end = p->s.cface ? reinterpret_cast<char*>(p->s.cface + L0.N) : reinterpret_cast<char*>(p->s.cnt + L0.V);
         zero_async(p->st, (size_t)(end - reinterpret_cast<char*>(p->st)), str);
