@@ -42,11 +42,11 @@ sys.path.insert(0, HERE)
 HBM_FALLBACK_GBS = 6650.0
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unit of work of a
-# kernel, from an ncu capture of a smaller mesh of the same kind
-# (profiles/k_pp_mixed384_slak.txt: k_pp of the last level,
-# SLAK, per quad of the level it refines, this build); times the units of the
-# bench's launch.
-TRAFFIC_PER_UNIT = {("k_pp", "slak", "last"): 145.0}
+# kernel, from one single-pass ncu capture of the bench workload itself
+# (profiles/launches_mixed512_slak.txt, launches_mixed512_lak.txt: k_pp of the
+# last level, per quad of the level it refines); times the units of the bench's
+# launch.
+TRAFFIC_PER_UNIT = {("k_pp", "slak", "last"): 147.73, ("k_pp", "lak", "last"): 233.53}
 # B200 HBM3e datasheet bandwidth (DGX figure), reported beside the measured peak
 HBM_NOMINAL_GBS = 8000.0
 
@@ -300,7 +300,7 @@ def run_ours(args, dist, rank, ws):
     if tpu is not None:
         units = stats[kern["level"]]["nfaces"]
         kern["traffic"] = tpu * units
-        kern["traffic_note"] = (f"{tpu} B per quad refined (ncu capture of a 384x384 mesh of this kind) x {units} quads; "
+        kern["traffic_note"] = (f"{tpu} B per quad refined (ncu, one pass, mixed512 capture) x {units} quads; "
                                 f"{tpu * units / kern['algorithmic_bytes_per_launch']:.2f}x the algorithmic bytes")
 
     # ms per level: the per-kernel event times summed by level, with the level's
@@ -670,7 +670,7 @@ def run_batch(args, torch, dist, rank, ws):
            "speedup_vs_plan_loop": plan_ms / batch_ms,
            "waves": b.waves, "groups": b.groups, "launches_per_execution": b.launches,
            "create_s": create_s, "generate_s": gen_s, "clocks": clk.summary(),
-           "plain": "slak_subdivide per mesh (allocates and frees its output per call)",
+           "plain": "slak_subdivide and slak_mesh_free per mesh (output arrays kept idle serve later calls)",
            "plan_loop": "per mesh: plan created untimed, one eager execution timed with CUDA events",
            "batched": "slak_batch, one CUDA graph per execution"}
     b.close()                                            # its outputs go before the one-call form's arrive
@@ -690,7 +690,7 @@ def run_batch(args, torch, dist, rank, ws):
         lib.slak_mesh_free(ctypes.byref(res[i]))     # elements share the array's memory
     out.update({"one_call_ms": one_ms, "one_call_value": faces * ws / (one_ms * 1e-3),
                 "speedup_one_call_vs_plain": plain_ms / one_ms,
-                "one_call": "slak_subdivide_batched: batch creation, per-mesh cudaMalloc of the outputs, one eager "
+                "one_call": "slak_subdivide_batched: batch creation, per-mesh output arrays (kept idle or new), one eager "
                             "execution (wall clock)"})
     return out
 

@@ -10,7 +10,7 @@
 //                atomic that counts the vertex's corners (low half) and owned
 //                edges (high half) at once; CAP: the corner's record into its
 //                vertex's bucket of 8, else its arrival rank
-//   k_c0_scan*   both counts' offsets: columns (sptr) and edge ids (eptr)
+//   k_c0_sums, k_c0_offsets   both counts' offsets: columns (sptr), edge ids (eptr)
 //   k_c0_bucket  (not CAP) the corners' records into their columns
 //   k_c0_verts   per vertex: its column sorted by corner, twins, edge ids of its
 //                owned edges, corner -> slot / twin, its vertex point
@@ -26,11 +26,12 @@
 // Why: these passes move little (about 100 MB at 1 M corners) and are bound by
 // the latency of dependent launches and gathers, so fewer passes is what
 // counts.  Measured on B200, launch by launch: 243,905 polygons (1 M corners)
-// 163 -> 97 us, 400,000 triangles in scattered order (LAK) 250 -> 119 us; whole
-// plans: 32x32 torus, 3 levels 39.5 -> 26.2 us, 1280 triangles, 4 levels
-// 81.8 -> 55.7 us, the scattered triangles, 1 level 200 -> 107 us.  CAP needs 128
-// bytes per vertex, so it stays with valences up to 8; above that the compact
-// records of the bucket pass serve every valence.
+// 163 -> 98 us, 400,000 triangles in scattered order (LAK) 250 -> 115 us; whole
+// plans of one level: the scattered triangles 200 -> 107 us, 128x128 torus 28 -> 17
+// us.  CAP needs 128 bytes per vertex, so it stays with valences up to 8; above
+// that the compact records of the bucket pass serve every valence.  One level with
+// CAP and, for the same meshes, without: 32x32 torus 12.8 and 14.9 us, 512x512
+// torus 44.2 and 49.6, 512x512 mixed torus 63.9 and 65.9 (SLAK; LAK 67.4 and 68.2).
 #pragma once
 
 #include "general.cuh"
@@ -47,7 +48,8 @@ __device__ __forceinline__ unsigned long long c0_count(int v, int w)
     return 1ull | ((unsigned long long)(LAK ? w < v : v < w) << 32);
 }
 
-// One face's corners c = b..e-1 with vertices vs(i): counts, records / ranks.
+// Corner c of face f (vertex v, next vertex w, previous u): its vertex's counts, its
+// record (CAP) or arrival rank.
 template <bool LAK, bool CAP>
 __device__ __forceinline__ void c0_corner(int c, int f, int v, int w, int u, bool first, int V,
                                           unsigned long long* __restrict__ cnt, int* __restrict__ rank,
@@ -246,7 +248,10 @@ struct k_c0_sums_g {
 
 // Each block adds up the tiles before its own (DIRECT, up to kC0Direct tiles:
 // from the counts themselves, one launch instead of two), then scans its tile.
-// Block 0 also checks the totals against the plan's corners and edges.
+// Block 0 also checks the totals against the plan's corners and edges.  One level
+// of a torus, by its tiles, with and without the counts themselves: 2 tiles 14.8
+// and 16.6 us, 4 16.9 and 16.7 (SLAK; with their state 18.1 and 16.8), 16 23.0 and
+// 16.9.
 constexpr int kC0Direct = 4;
 template <bool DIRECT>
 __device__ __forceinline__ void k_c0_offsets_body(const unsigned bx_, const u64* __restrict__ cnt, int n,

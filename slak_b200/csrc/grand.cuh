@@ -112,7 +112,12 @@ __device__ __forceinline__ float4 ep_lak(float4 a, float4 e, float4 f0, float4 f
 // The vertex point of PP's face point f (position Pf) of a polygon face with
 // corners fb..fe-1, at most kPpFace of them: its column is the corners 4j + 2,
 // ascending, each C quad {f, c(j), g(j), c(next j)}.  Formulas and order of
-// g3_vertex.
+// g3_vertex.  Longer faces leave records for k_g3.  3 levels, B200, with the line
+// at 4, 8 and 16 corners: faces of 9 (5,000 prisms) SLAK 105, 105, 109 us, LAK 125,
+// 125, 137; of 12 (4,000) 112, 112, 120 and 137, 137, 154; of 6 (6,000) 82, 83, 84
+// and 89, 94, 94; of 8 (5,000) 90, 88, 88 and 102, 113, 113; 512x512 mixed torus 321,
+// 321, 320 and 368, 382, 383.  (SLAK is indifferent below 8; LAK, whose tails are
+// selected one by one here, is better off with 4.)
 constexpr int kPpFace = 8;
 template <bool LAK>
 __device__ __forceinline__ float4 pp_face_vertex(const FastDims& d, const int4* __restrict__ pids,

@@ -230,7 +230,8 @@ void launch_fast_gq(const Level& Pl, const Level& L, bool lak, bool comp, Lc& lc
 #elif SLAK_UNIT == 4
 // Level 1 of a closed polygon input (poly1.cuh): C = L, its parent Pl the
 // input.  k_p1 runs blocks of bs[0] / 2 threads; bs[1] picks its register cap
-// (128, 256, 512: for 1024, 768, 512 resident threads).
+// (128, 256, 512: for 1024, 768, 512 resident threads).  Bulk-copied records: as
+// launch_fast_t's.
 template <bool LAK, bool STATE>
 static void launch_p1_t(const Level& Pl, const Level& L, Faces<false> pf, bool comp, Lc& lc)
 {
