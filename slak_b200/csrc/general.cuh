@@ -120,7 +120,7 @@ __device__ __forceinline__ void k_valence_hist_body(const unsigned bx_, int V, c
     if (threadIdx.x < 17) h[threadIdx.x] = 0;
     __syncthreads();
     const int v = bx_ * blockDim.x + threadIdx.x;
-    if (v < V) atomicAdd(&h[min(sptr[v + 1] - sptr[v], 16)], 1);
+    if (v < V) atomicAdd(&h[max(0, min(sptr[v + 1] - sptr[v], 16))], 1);
     __syncthreads();
     if (threadIdx.x < 17 && h[threadIdx.x]) atomicAdd(hist + threadIdx.x, h[threadIdx.x]);
 }
@@ -142,7 +142,9 @@ struct k_valence_hist_g {
 // `loose`); k_vsort makes it canonical.  A malformed polygon mesh (a face the
 // valence pass rejected, or corners past ptr[F]) brings more corners to a
 // vertex than its column counts: those find no slot (r < 0) and are dropped,
-// so nothing is written outside the column; the level fails with BAD_MESH.
+// so nothing is written outside the column; the level fails with BAD_MESH.  Faces
+// that overlap (offsets that descend somewhere) count more than N corners: the
+// columns' offsets end at N (the scan's cap) and no corner is placed past it.
 __device__ __forceinline__ void k_bucket_body(const unsigned bx_, const int* __restrict__ ids, int N, int V, const int* __restrict__ sptr,
                                               int* __restrict__ fill, int* __restrict__ loose)
 {
@@ -151,7 +153,7 @@ __device__ __forceinline__ void k_bucket_body(const unsigned bx_, const int* __r
     int v = ids[c];
     if ((unsigned)v >= (unsigned)V) return;
     int r = atomicSub(fill + v, 1) - 1;
-    if (r >= 0) loose[sptr[v] + r] = c;
+    if (r >= 0 && (unsigned)sptr[v] + (unsigned)r < (unsigned)N) loose[sptr[v] + r] = c;
 }
 __global__ void k_bucket(const int* __restrict__ ids, int N, int V, const int* __restrict__ sptr,
                          int* __restrict__ fill, int* __restrict__ loose)
@@ -175,12 +177,16 @@ struct k_bucket_g {
 // `xslot` the slot of every corner is exported as well (corner -> slot, for
 // the fast path).
 template <bool QUAD>
-__device__ __forceinline__ void vsort_neighbours(Faces<QUAD> fc, const int* __restrict__ ids, int s, int c,
+__device__ __forceinline__ void vsort_neighbours(Faces<QUAD> fc, const int* __restrict__ ids, int N, int s, int c,
                                                  int* __restrict__ snext, int* __restrict__ sprev,
                                                  int* __restrict__ sprevc)
 {
-    const int p = fc.prev(c);
-    snext[s] = __ldg(ids + fc.next(c));
+    int p = fc.prev(c), q = fc.next(c);
+    if (!QUAD) {            // (a corner of no accepted face has no neighbours: itself)
+        if ((unsigned)p >= (unsigned)N) p = c;
+        if ((unsigned)q >= (unsigned)N) q = c;
+    }
+    snext[s] = __ldg(ids + q);
     sprev[s] = __ldg(ids + p);
     sprevc[s] = p;
 }
@@ -212,7 +218,7 @@ __device__ __forceinline__ void k_vsort_body(const unsigned bx_, Faces<QUAD> fc,
     if (r >= n) return;
     sc[b + r] = c;
     if (xslot) xslot[c] = b + r;
-    vsort_neighbours(fc, ids, b + r, c, snext, sprev, sprevc);
+    vsort_neighbours(fc, ids, N, b + r, c, snext, sprev, sprevc);
 }
 template <bool QUAD>
 __global__ void k_vsort(Faces<QUAD> fc, const int* __restrict__ ids, int N, int V, const int* __restrict__ sptr,

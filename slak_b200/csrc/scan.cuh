@@ -2,7 +2,7 @@
 //
 // Replaces CubFunctions::scan_exclusive (LibInclude/device/cub_wrappers.cuh:30-43):
 // out[0] = 0, out[i+1] = in[0] + ... + in[i], out has n+1 entries, so out[n] is
-// the total.  Reduce-then-scan over tiles of 2048 items: tile sums, one block
+// the total; no output exceeds `cap` (a wrapped sum counts as above it).  Reduce-then-scan over tiles of 2048 items: tile sums, one block
 // scanning the tile sums, then a tile scan with the tile's carry (up to 2048
 // tiles, each tile's block sums the tile sums before it instead).  Integer and
 // deterministic.
@@ -105,7 +105,8 @@ struct k_scan_tiles_g {
 };
 
 __device__ __forceinline__ void k_scan_final_body(const unsigned bx_, const int* __restrict__ in, int64_t n,
-                                                  const int* __restrict__ tsum, int nt, int* __restrict__ out)
+                                                  const int* __restrict__ tsum, int nt, int* __restrict__ out,
+                                                  unsigned cap)
 {
     __shared__ int tile[kScanTile];
     __shared__ int tot;
@@ -129,15 +130,16 @@ __device__ __forceinline__ void k_scan_final_body(const unsigned bx_, const int*
     for (int i = 0; i < kScanItems; ++i) {
         int j = i * kBlock + threadIdx.x;
         int64_t k = base + j;
-        if (k < n) out[k] = tile[j];
+        if (k < n) out[k] = (int)min((unsigned)tile[j], cap);
     }
-    if (bx_ == 0 && threadIdx.x == 0) out[n] = tsum[nt];
+    if (bx_ == 0 && threadIdx.x == 0) out[n] = (int)min((unsigned)tsum[nt], cap);
 }
 __global__ void __launch_bounds__(kBlock) k_scan_final(const int* __restrict__ in, int64_t n,
-                                                       const int* __restrict__ tsum, int nt, int* __restrict__ out)
+                                                       const int* __restrict__ tsum, int nt, int* __restrict__ out,
+                                                       unsigned cap)
 {
     griddep_enter();
-    k_scan_final_body(blockIdx.x, in, n, tsum, nt, out);
+    k_scan_final_body(blockIdx.x, in, n, tsum, nt, out, cap);
 }
 struct k_scan_final_g {
     static constexpr int kBounds = 1, kMaxT = kBlock, kMinB = 0;
@@ -154,7 +156,7 @@ constexpr int kScanSmallTiles = 2048;
 
 __device__ __forceinline__ void k_scan_final_small_body(const unsigned bx_, const int* __restrict__ in, int64_t n,
                                                         const int* __restrict__ tsum, int nt,
-                                                        int* __restrict__ out)
+                                                        int* __restrict__ out, unsigned cap)
 {
     __shared__ int tile[kScanTile];
     __shared__ int tot;
@@ -191,16 +193,16 @@ __device__ __forceinline__ void k_scan_final_small_body(const unsigned bx_, cons
     for (int i = 0; i < kScanItems; ++i) {
         int j = i * kBlock + threadIdx.x;
         int64_t k = base + j;
-        if (k < n) out[k] = tile[j];
+        if (k < n) out[k] = (int)min((unsigned)tile[j], cap);
     }
-    if (bx_ == 0 && threadIdx.x == 0) out[n] = total;
+    if (bx_ == 0 && threadIdx.x == 0) out[n] = (int)min((unsigned)total, cap);
 }
 __global__ void __launch_bounds__(kBlock) k_scan_final_small(const int* __restrict__ in, int64_t n,
                                                              const int* __restrict__ tsum, int nt,
-                                                             int* __restrict__ out)
+                                                             int* __restrict__ out, unsigned cap)
 {
     griddep_enter();
-    k_scan_final_small_body(blockIdx.x, in, n, tsum, nt, out);
+    k_scan_final_small_body(blockIdx.x, in, n, tsum, nt, out, cap);
 }
 struct k_scan_final_small_g {
     static constexpr int kBounds = 1, kMaxT = kBlock, kMinB = 0;
@@ -214,18 +216,19 @@ struct k_scan_final_small_g {
 inline int64_t scan_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
 // tmp must hold scan_tiles(n) + 1 ints
-inline void scan_exclusive(const int* in, int* out, int64_t n, int* tmp, cudaStream_t s, int64_t* launches)
+inline void scan_exclusive(const int* in, int* out, int64_t n, int* tmp, cudaStream_t s, int64_t* launches,
+                           unsigned cap = 0x7fffffffu)
 {
     int64_t nt = scan_tiles(n);
     if (nt < 1) nt = 1;
     launch_g<k_scan_reduce_g>((unsigned)nt, kBlock, s, in, n, tmp);
     if (nt <= kScanSmallTiles) {
-        launch_g<k_scan_final_small_g>((unsigned)nt, kBlock, s, in, n, tmp, (int)nt, out);
+        launch_g<k_scan_final_small_g>((unsigned)nt, kBlock, s, in, n, tmp, (int)nt, out, cap);
         if (launches) *launches += 2;
         return;
     }
     launch_g<k_scan_tiles_g>(1, kBlock, s, tmp, (int)nt);
-    launch_g<k_scan_final_g>((unsigned)nt, kBlock, s, in, n, tmp, (int)nt, out);
+    launch_g<k_scan_final_g>((unsigned)nt, kBlock, s, in, n, tmp, (int)nt, out, cap);
     if (launches) *launches += 3;
 }
 

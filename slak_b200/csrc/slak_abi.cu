@@ -431,7 +431,7 @@ void launch_topology_a(const Level& L, int li, int scheme, Scratch& s, DevStatus
         lc.after("k_valence");
     }
     int64_t dummy = 0;
-    scan_exclusive(s.cnt, s.sptr, V, s.tmp, str, &dummy);
+    scan_exclusive(s.cnt, s.sptr, V, s.tmp, str, &dummy, (unsigned)N);
     lc.after("scan(valence)", 3);
     // the unsorted columns live in sflag until k_edges writes the flags
     launch_g<k_bucket_g>(grid_for(N), kBlock, str, L.ids, N, V, s.sptr, s.cnt, s.sflag);
